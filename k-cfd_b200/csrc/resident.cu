@@ -1,0 +1,144 @@
+// On-chip BiCGSTAB of small systems: kernels and launches (design in resident.cuh).
+#include "resident.cuh"
+
+#include <algorithm>
+#include <cstring>
+#include <mutex>
+#include <type_traits>
+
+namespace kcfd {
+namespace res {
+
+template <int NRHS, int PREC, int R>
+__global__ void __launch_bounds__(kBlock, 1) k_resident(SolveArgs a, int width) {
+    extern __shared__ __align__(16) char store[];
+    __shared__ Shared sh;
+    Team tm;
+    int id;
+    cluster_ids(tm.rank, tm.size, id);
+    tm.sh = &sh;
+    tm.budget = a.ctl.budget;
+    tm.init();
+    solve_on_chip<NRHS, PREC, R>(tm, a, width, store);
+    tm.sync();  // no CTA leaves while another may still gather from it
+}
+
+namespace {
+
+// f(NRHS, PREC, R) as template arguments; false for a combination that is not compiled (more
+// vectors than registers).
+template <class F>
+bool dispatch(int nrhs, int precond, int r, F f) {
+#define KC_RES(N, P, RR)                                                                                   \
+    if (nrhs == N && precond == P && r == RR) {                                                            \
+        f(std::integral_constant<int, N>(), std::integral_constant<int, P>(), std::integral_constant<int, RR>()); \
+        return true;                                                                                       \
+    }
+#define KC_RES_P(N, RR) KC_RES(N, 0, RR) KC_RES(N, 1, RR) KC_RES(N, 2, RR)
+    KC_RES_P(1, 1) KC_RES_P(1, 2) KC_RES_P(1, 4) KC_RES_P(1, 8)
+    KC_RES_P(2, 1) KC_RES_P(2, 2) KC_RES_P(2, 4)
+    KC_RES_P(3, 1) KC_RES_P(3, 2)
+#undef KC_RES_P
+#undef KC_RES
+    return false;
+}
+
+void* kernel_of(int nrhs, int precond, int r) {
+    void* k = nullptr;
+    dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { k = (void*)k_resident<n(), p(), rr()>; });
+    return k;
+}
+
+cudaLaunchConfig_t config(const Plan& p, cudaStream_t st, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(p.ctas);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = p.ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// What the device grants a kernel: dynamic shared memory, and the largest cluster that can be
+// resident at that much. Asked once per device and kernel (the questions take up to a
+// millisecond each).
+struct Limits {
+    int smem = 0, ctas = 0;
+};
+
+Limits limits(int nrhs, int precond, int r) {
+    constexpr int kDevices = 64;
+    static std::mutex mu;
+    static Limits known[kDevices][4][3][9];
+    int dev = 0;
+    void* f = kernel_of(nrhs, precond, r);
+    if (!f || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return Limits();
+    std::lock_guard<std::mutex> lock(mu);
+    Limits& L = known[dev][nrhs][precond][r];
+    if (L.smem > 0) return L;
+    int optin = 0;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return Limits();
+    }
+    Plan p;
+    p.smem = optin - (int)fa.sharedSizeBytes;
+    for (p.ctas = kMaxCtas; p.ctas > 1; p.ctas /= 2) {
+        int m = 0;
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = config(p, nullptr, at);
+        if (cudaOccupancyMaxActiveClusters(&m, f, &cfg) == cudaSuccess && m >= 1) break;
+        cudaGetLastError();
+    }
+    L.ctas = p.ctas;
+    L.smem = p.smem;
+    return L;
+}
+
+}  // namespace
+
+Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max_ctas) {
+    const int nlev = (int)lev.size() - 1;
+    if (width < 1 || width > 64 || nlev > 4096) return Plan();
+    // the fewest rows per thread first: a thread's rows are done one after another
+    for (int r = 1; r <= 8; r *= 2) {
+        const Limits L = limits(nrhs, precond, r);
+        size_t bytes = SIZE_MAX;
+        dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr()>::bytes(width, nlev); });
+        if (L.smem == 0 || bytes > (size_t)L.smem) continue;
+        for (int c = 1; c <= std::min(max_ctas, L.ctas); c *= 2) {
+            int64_t rows = 0;
+            for (int l = 0; l < nlev; ++l) rows += (lev[l + 1] - lev[l] + c - 1) / c;
+            if (rows > kBlock * r) continue;
+            Plan p;
+            p.ctas = c;
+            p.rows_per_thread = r;
+            p.width = width;
+            p.smem = (int)bytes;
+            return p;
+        }
+    }
+    return Plan();
+}
+
+cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, cudaStream_t st) {
+    SolveArgs args = a;
+    int width = p.width;
+    void* ptrs[] = {&args, &width};
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = config(p, st, at);
+    return cudaLaunchKernelExC(&cfg, kernel_of(nrhs, precond, p.rows_per_thread), ptrs);
+}
+
+}  // namespace res
+}  // namespace kcfd

@@ -1,0 +1,29 @@
+// Host interface of the on-chip BiCGSTAB (resident.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <vector>
+
+namespace kcfd {
+struct SolveArgs;
+namespace res {
+
+constexpr int kMaxCtas = 16;
+
+// Launch shape of an on-chip solve: one cluster of `ctas` CTAs, each thread with
+// `rows_per_thread` rows of at most `width` entries, `smem` bytes of shared memory per CTA.
+struct Plan {
+    int ctas = 0;  // 0: the system does not fit on chip
+    int rows_per_thread = 0, width = 0, smem = 0;
+};
+
+// Shape for a matrix of at most `width` entries a row whose levels start at rows lev[l]
+// (lev.back() rows), on up to max_ctas CTAs.
+Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max_ctas);
+
+// One FP64 solve; a holds the caller's pointers (x, b, outputs) and the handle's pattern,
+// values and preconditioner.
+cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, cudaStream_t st);
+
+}  // namespace res
+}  // namespace kcfd

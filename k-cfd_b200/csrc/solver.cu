@@ -27,6 +27,8 @@
 //    ranges, the lower part of a row is exactly its columns left of the diagonal, and
 //    the forward / backward sweeps read contiguous memory. b and x are permuted on
 //    entry and exit inside the same launch.
+//  * FP64 systems that fit the shared memory of a thread-block cluster (up to 32,768 rows)
+//    are solved there, when the team is chosen automatically (resident.cuh).
 //  * Large FP64 systems run on the graph engine instead (team 3, graph_engine.cuh):
 //    the same iteration as lean phase kernels in one CUDA graph with a device-side
 //    WHILE loop. A solve issued while its stream is being captured falls back to the
@@ -47,46 +49,10 @@
 #include "team.cuh"
 #include "amg.h"
 #include "graph_engine.cuh"
+#include "resident.h"
+#include "solve_args.h"
 
 namespace kcfd {
-
-constexpr double kEps2 = 4.930380657631324e-32;  // float64 eps^2 (scipy rhotol/omegatol)
-
-struct SolveArgs {
-    int n;
-    int lanes;
-    // matrix of the Krylov iterations (the level-permuted copy when perm != null)
-    const int* indptr;
-    const int* indices;
-    const double* vals64;
-    const float* vals32;
-    const int* perm;     // [n] permuted row -> caller row, or null
-    double* px;          // [n*nrhs] permuted FP64 solution (perm only)
-    double* pb;          // [n*nrhs] permuted FP64 rhs (perm only)
-    // preconditioner
-    void* dinv;          // Jacobi inverse diagonal, V
-    const int* diag;     // [n] position of the diagonal (ILU)
-    void* lu;            // [nnz] ILU factors, V
-    void* ludinv;        // [n] 1 / u_ii, V
-    const int* lev_ptr;  // [nlev+1] level row ranges
-    int nlev;
-    // vectors
-    void* work;          // 9 V vectors of n*nrhs
-    double* x;           // caller FP64 solution (x0 on entry)
-    const double* b;     // caller FP64 rhs
-    double* r64;         // MIXED outer residual
-    // control
-    int stop;
-    int maxiter;
-    int max_refine;
-    int inner_maxiter;
-    int max_restarts;    // KCFD_STOP_SCIPY: restarts on rho / omega breakdown (0: scipy's stop)
-    double rtol, atol, inner_rtol;
-    int* iters_out;
-    double* relres_out;
-    int* status_out;
-    TeamCtl ctl;
-};
 
 template <typename V>
 struct Vecs {
@@ -704,9 +670,6 @@ __device__ void permute_out(Team& tm, const SolveArgs& a) {
     });
 }
 
-// Verification passes of a batched FP64 solve (see solve_fp64).
-constexpr int kVerifyPasses = 3;
-
 // FP64 solve.
 template <int NRHS, int PREC, class Team>
 __device__ void solve_fp64(Team& tm, const SolveArgs& a, double* smem) {
@@ -1264,6 +1227,7 @@ struct kcfd_solver {
     void* ludinv = nullptr;
     // KCFD_PREC_AMG: the multigrid hierarchy (graph engine only)
     kcfd_amg* amg = nullptr;
+    res::Plan res;  // on-chip solve (ctas > 0), in place of the persistent kernel
     // team control
     unsigned int* bar = nullptr;
     double* partials = nullptr;
@@ -2096,10 +2060,13 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
         }
     }
     // team and launch shape
-    // auto: one CTA for tiny systems; the persistent grid kernel up to 40,000 unknowns
-    // (and for every mixed solve); the graph engine for large FP64 systems. Measured on
-    // a 4,096-row p' system: one CTA 35 us per Krylov iteration, the grid kernel 18 us,
-    // the graph engine 25 us. A caller that runs many small solves concurrently (the
+    // auto: up to 40,000 unknowns FP64 systems that fit run on chip (resident.cuh, below);
+    // the others, and every mixed solve, on one CTA (tiny systems) or the persistent grid
+    // kernel; the graph engine takes the larger FP64 systems. Measured per Krylov iteration
+    // (Jacobi, one right-hand side, 64^2 cavity p'): one CTA 28 us, the grid kernel 20 us,
+    // the graph engine 25 us, on chip 3.9 us (16 CTAs, one row a thread); with ILU(0) on a
+    // 7,200-triangle channel 40 us on the grid kernel, 6.9 us on chip; 32,400 rows (8 rows
+    // a thread) 7.1 us on chip. A caller that runs many small solves concurrently (the
     // served loop) asks for one CTA explicitly, so that they overlap.
     int team = (amg || cg) ? 3 : opts->team;
     if (team == 0) {
@@ -2273,6 +2240,15 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     } else {
         s->grid = 1;
     }
+    // On chip where it fits: FP64 systems below the graph engine's line, unless the caller
+    // asked for a launch shape (lanes, block, the grid team); one that asked for one CTA
+    // gets one.
+    if (!mixed && team <= 2 && opts->team <= 1 && opts->lanes <= 0 && opts->block <= 0) {
+        const std::vector<int>& rp = s->perm ? pip : ip;
+        int width = 0;
+        for (int i = 0; i < n; ++i) width = std::max(width, rp[i + 1] - rp[i]);
+        s->res = res::plan(width, nrhs, opts->precond, lptr, opts->team == 1 ? 1 : res::kMaxCtas);
+    }
     const size_t len = (size_t)n * nrhs;
     bool ok = upload(&s->lev_ptr, lptr);
     ok = ok && cudaMalloc(&s->work, 9 * len * vsz) == cudaSuccess;
@@ -2391,6 +2367,10 @@ int kcfd_solver_solve(kcfd_solver* s, const kcfd_csr_t* A, const double* b, doub
             return ge_solve(s, A, b, x, iters, relres, status, (cudaStream_t)stream);
         KCFD_REQUIRE(s->o.precond != KCFD_PREC_AMG,
                      "kcfd_solver_solve: an AMG solve runs as its own graph; issue it outside stream capture");
+    }
+    if (s->res.ctas > 0) {
+        KCFD_CUDA(res::solve(s->res, s->o.nrhs, s->o.precond, a, (cudaStream_t)stream));
+        return KCFD_OK;
     }
     void* kern = solve_kernel_ptr(mixed, s->o.nrhs, s->o.precond, s->team >= 2, s->block);
     KCFD_REQUIRE(kern != nullptr, "kcfd_solver_solve: no kernel for this configuration");
