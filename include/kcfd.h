@@ -323,7 +323,10 @@ void kcfd_amg_destroy(kcfd_amg* h);
  * 2 CTAs for systems of at least 8R, 4R or 2R rows, R = cluster_rows (0: 16384), so
  * that the big systems get CTAs in proportion to their size; or one tier of
  * cluster_size CTAs from cluster_rows rows (0: 131072). Then systems of at least
- * big_rows rows are solved by one 512-thread CTA, the rest by one 256-thread CTA. A
+ * big_rows rows are solved by one 512-thread CTA, the rest by one 256-thread CTA. With
+ * cluster_rows, cluster_size and big_rows all 0 and lanes <= 1, FP64 systems that fit the
+ * shared memory of a cluster (up to 32,768 rows) are solved on chip by the fewest CTAs
+ * that hold them, whatever tier their size gives them. A
  * system's tier depends only on its own size (and on whether a cluster of its size
  * can be resident at all), so its result is the same alone and in any mix. No
  * counterpart API in the reference, which solves one system per call

@@ -23,6 +23,24 @@ __global__ void __launch_bounds__(kBlock, 1) k_resident(SolveArgs a, int width) 
     tm.sync();  // no CTA leaves while another may still gather from it
 }
 
+// Systems B.order[first + cluster index]: independent solves, one cluster each, scheduled by
+// the hardware as SMs become free.
+template <int PREC, int R>
+__global__ void __launch_bounds__(kBlock, 1) k_resident_batch(BatchArgs B, int first, int width, long long budget) {
+    extern __shared__ __align__(16) char store[];
+    __shared__ Shared sh;
+    Team tm;
+    int id;
+    cluster_ids(tm.rank, tm.size, id);
+    tm.sh = &sh;
+    tm.budget = budget;
+    tm.init();
+    SolveArgs a = batch_args<double>(B, B.order[first + id]);
+    a.dinv = nullptr;
+    solve_on_chip<1, PREC, R>(tm, a, width, store);
+    tm.sync();
+}
+
 namespace {
 
 // f(NRHS, PREC, R) as template arguments; false for a combination that is not compiled (more
@@ -35,7 +53,7 @@ bool dispatch(int nrhs, int precond, int r, F f) {
         return true;                                                                                       \
     }
 #define KC_RES_P(N, RR) KC_RES(N, 0, RR) KC_RES(N, 1, RR) KC_RES(N, 2, RR)
-    KC_RES_P(1, 1) KC_RES_P(1, 2) KC_RES_P(1, 4) KC_RES_P(1, 8)
+    KC_RES_P(1, 1) KC_RES_P(1, 2) KC_RES_P(1, 3) KC_RES_P(1, 4) KC_RES_P(1, 6) KC_RES_P(1, 8)
     KC_RES_P(2, 1) KC_RES_P(2, 2) KC_RES_P(2, 4)
     KC_RES_P(3, 1) KC_RES_P(3, 2)
 #undef KC_RES_P
@@ -43,16 +61,22 @@ bool dispatch(int nrhs, int precond, int r, F f) {
     return false;
 }
 
-void* kernel_of(int nrhs, int precond, int r) {
+void* kernel_of(int nrhs, int precond, int r) {  // nrhs 0: the batched kernel
     void* k = nullptr;
+    if (nrhs == 0) {
+        dispatch(1, precond, r, [&](auto, auto p, auto rr) {
+            if constexpr (p() != KCFD_PREC_ILU0) k = (void*)k_resident_batch<p(), rr()>;
+        });
+        return k;
+    }
     dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { k = (void*)k_resident<n(), p(), rr()>; });
     return k;
 }
 
-cudaLaunchConfig_t config(const Plan& p, cudaStream_t st, cudaLaunchAttribute* at) {
+cudaLaunchConfig_t config(const Plan& p, cudaStream_t st, cudaLaunchAttribute* at, int clusters = 1) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(p.ctas);
+    cfg.gridDim = dim3(p.ctas * clusters);
     cfg.blockDim = dim3(kBlock);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
@@ -111,12 +135,12 @@ Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max
     const int nlev = (int)lev.size() - 1;
     if (width < 1 || width > 64 || nlev > 4096) return Plan();
     // the fewest rows per thread first: a thread's rows are done one after another
-    for (int r = 1; r <= 8; r *= 2) {
+    for (int r = 1; r <= 8; ++r) {
         const Limits L = limits(nrhs, precond, r);
         size_t bytes = SIZE_MAX;
         dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr()>::bytes(width, nlev); });
         if (L.smem == 0 || bytes > (size_t)L.smem) continue;
-        for (int c = 1; c <= std::min(max_ctas, L.ctas); c *= 2) {
+        for (int c = 1; c <= std::min(max_ctas, L.ctas); ++c) {
             int64_t rows = 0;
             for (int l = 0; l < nlev; ++l) rows += (lev[l + 1] - lev[l] + c - 1) / c;
             if (rows > kBlock * r) continue;
@@ -129,6 +153,35 @@ Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max
         }
     }
     return Plan();
+}
+
+Plan plan_compact(int n, int width, int precond) {
+    if (width < 1 || width > 64 || precond < 0 || precond > 1) return Plan();
+    // two CTAs or more hold over 1,024 rows each; odd large counts are rounded up, which
+    // leaves fewer shapes (launches) in a batch
+    for (int c = 1; c <= kMaxCtas; c += c < 6 ? 1 : c < 12 ? 2 : 4)
+        for (int r = c < 3 ? 1 : 8; r <= 8; ++r) {
+            const Limits L = limits(0, precond, r);
+            const size_t bytes = (size_t)kBlock * r * (8 + 12 * (size_t)width) + 16;
+            if (L.ctas < c || bytes > (size_t)L.smem || (int64_t)c * kBlock * r < n) continue;
+            Plan p;
+            p.ctas = c;
+            p.rows_per_thread = r;
+            p.width = width;
+            p.smem = (int)bytes;
+            return p;
+        }
+    return Plan();
+}
+
+cudaError_t batch(const Plan& p, const BatchArgs& B, int first, int count, cudaStream_t st) {
+    BatchArgs args = B;
+    int width = p.width;
+    long long budget = 4000000000LL;  // ~2 s at 2 GHz per wait
+    void* ptrs[] = {&args, &first, &width, &budget};
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = config(p, st, at, count);
+    return cudaLaunchKernelExC(&cfg, kernel_of(0, B.precond, p.rows_per_thread), ptrs);
 }
 
 cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, cudaStream_t st) {

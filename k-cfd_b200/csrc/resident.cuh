@@ -5,7 +5,7 @@
 // software barrier there (20 us per iteration on the 64^2 cavity's p' system, whose 0.5 MB
 // take 0.1 us at HBM rate). Here everything stays in a cluster of 1 to 16 CTAs of 256
 // threads for the whole solve:
-//  * a thread owns R rows (1, 2, 4 or 8) and keeps their Krylov vectors in registers; R is
+//  * a thread owns R rows (1 to 8) and keeps their Krylov vectors in registers; R is
 //    a template argument, so the vector phases have no loops and no address arithmetic. 256
 //    threads leave 255 registers for it, and fewer warps make the block reductions cheaper;
 //  * the matrix and the preconditioner lie in shared memory, entry-major ([entry][local
@@ -341,6 +341,7 @@ struct System {
             int li = -1;
             const int i = row_of(tm, t, li);
             const int kb = i >= 0 ? __ldg(a.indptr + i) : 0, len = i >= 0 ? __ldg(a.indptr + i + 1) - kb : 0;
+            double d = 0.0;
 #pragma unroll 4
             for (int k = 0; k < width; ++k) {
                 uint32_t adr = remote(v0 + 8 * NRHS * t, tm.rank);  // padding: the own row, value 0
@@ -349,6 +350,7 @@ struct System {
                     const int j = __ldg(a.indices + kb + k);
                     v = a.vals64[kb + k];
                     if (PREC == KCFD_PREC_ILU0) f = lu[kb + k];
+                    if (PREC == KCFD_PREC_JACOBI && j == i) d += v;
                     const int l = nlev == 1 ? 0 : level_of(s.lev, nlev, j);
                     const int per = s.loc[l + 1] - s.loc[l];
                     const int at = j - s.lev[l], rk = at / per;
@@ -361,7 +363,8 @@ struct System {
             di[u] = 0.0;
             lv[u] = -1;
             dk[u] = 0;
-            if (i >= 0 && PREC == KCFD_PREC_JACOBI) di[u] = ((const double*)a.dinv)[i];
+            if (i >= 0 && PREC == KCFD_PREC_JACOBI)  // batched systems are set up here
+                di[u] = a.dinv ? ((const double*)a.dinv)[i] : (fabs(d) > 1e-30 ? 1.0 / d : 0.0);
             if (i >= 0 && PREC == KCFD_PREC_ILU0) {
                 di[u] = ((const double*)a.ludinv)[i];
                 lv[u] = li;

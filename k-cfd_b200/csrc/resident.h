@@ -6,6 +6,7 @@
 
 namespace kcfd {
 struct SolveArgs;
+struct BatchArgs;
 namespace res {
 
 constexpr int kMaxCtas = 16;
@@ -21,9 +22,16 @@ struct Plan {
 // (lev.back() rows), on up to max_ctas CTAs.
 Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max_ctas);
 
+// Shape on the fewest CTAs that hold a system of n rows (Jacobi or no preconditioner, one
+// right-hand side).
+Plan plan_compact(int n, int width, int precond);
+
 // One FP64 solve; a holds the caller's pointers (x, b, outputs) and the handle's pattern,
 // values and preconditioner.
 cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, cudaStream_t st);
+
+// Systems B.order[first .. first + count) of a batch, each by a cluster of its own.
+cudaError_t batch(const Plan& p, const BatchArgs& B, int first, int count, cudaStream_t st);
 
 }  // namespace res
 }  // namespace kcfd

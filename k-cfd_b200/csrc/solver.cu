@@ -934,35 +934,6 @@ __global__ void jacobi_apply_kernel(int n, const double* __restrict__ dinv, cons
 // FP32 difference-form operator row by row, and solves it alone (CtaTeam: block
 // barriers and block reductions only, no inter-CTA waits). A system's result does not
 // depend on which CTA ran it or on what ran beside it.
-struct BatchSys {
-    int n, nnz;
-    long long row_off;  // rows before this system in the packed vectors
-    long long ptr_off;  // offset of its (n + 1) row pointers
-    long long nnz_off;  // offset of its entries
-};
-
-struct BatchArgs {
-    int nsys, lanes, mixed, precond, stop, maxiter, max_refine, inner_maxiter, max_restarts;
-    int nq;  // systems in this launch's queue (order[0..nq))
-    double rtol, atol, inner_rtol;
-    const BatchSys* sys;
-    const int* order;
-    int* queue;
-    const int* indptr;
-    const int* indices;
-    const double* vals64;
-    float* vals32;
-    void* dinv;
-    int* lev;
-    void* work;
-    double* r64;
-    double* x;
-    const double* b;
-    int* iters;
-    double* relres;
-    int* status;
-};
-
 template <typename V>
 __device__ void batch_prep(const BatchArgs& B, const BatchSys& S, int sid, V* dinv, float* v32, bool mixed) {
     const int* ip = B.indptr + S.ptr_off;
@@ -994,43 +965,11 @@ __device__ void batch_prep(const BatchArgs& B, const BatchSys& S, int sid, V* di
 template <int MIXED>
 __global__ void batch_prep_kernel(BatchArgs B) {
     using V = typename std::conditional<MIXED, float, double>::type;
-    for (int sid = blockIdx.x; sid < B.nsys; sid += gridDim.x) {
+    for (int q = blockIdx.x; q < B.nq; q += gridDim.x) {
+        const int sid = B.order[q];
         const BatchSys S = B.sys[sid];
         batch_prep<V>(B, S, sid, (V*)B.dinv + S.row_off, B.vals32 ? B.vals32 + S.nnz_off : nullptr, MIXED);
     }
-}
-
-// SolveArgs of system sid of a batch (everything but the team control).
-template <typename V>
-__device__ SolveArgs batch_args(const BatchArgs& B, int sid) {
-    const BatchSys S = B.sys[sid];
-    SolveArgs a;
-    memset(&a, 0, sizeof(a));
-    a.n = S.n;
-    a.lanes = B.lanes;
-    a.indptr = B.indptr + S.ptr_off;
-    a.indices = B.indices + S.nnz_off;
-    a.vals64 = B.vals64 + S.nnz_off;
-    a.vals32 = B.vals32 ? B.vals32 + S.nnz_off : nullptr;
-    a.dinv = (V*)B.dinv + S.row_off;
-    a.lev_ptr = B.lev + 2 * sid;
-    a.nlev = 1;
-    a.work = (V*)B.work + 9 * S.row_off;
-    a.x = B.x + S.row_off;
-    a.b = B.b + S.row_off;
-    a.r64 = B.r64 ? B.r64 + S.row_off : nullptr;
-    a.stop = B.stop;
-    a.maxiter = B.maxiter;
-    a.max_refine = B.max_refine;
-    a.inner_maxiter = B.inner_maxiter;
-    a.max_restarts = B.max_restarts;
-    a.rtol = B.rtol;
-    a.atol = B.atol;
-    a.inner_rtol = B.inner_rtol;
-    a.iters_out = B.iters + sid;
-    a.relres_out = B.relres + sid;
-    a.status_out = B.status + sid;
-    return a;
 }
 
 // Team control of the cluster tier: per cluster a barrier counter, a published queue
@@ -2242,12 +2181,14 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     }
     // On chip where it fits: FP64 systems below the graph engine's line, unless the caller
     // asked for a launch shape (lanes, block, the grid team); one that asked for one CTA
-    // gets one.
-    if (!mixed && team <= 2 && opts->team <= 1 && opts->lanes <= 0 && opts->block <= 0) {
+    // gets one (256 threads, a lane a row: also by those numbers).
+    const bool auto_shape = opts->team == 0 && opts->lanes <= 0 && opts->block <= 0;
+    const bool one_cta = opts->team == 1 && opts->lanes <= 1 && (opts->block <= 0 || opts->block == 256);
+    if (!mixed && team <= 2 && (auto_shape || one_cta)) {
         const std::vector<int>& rp = s->perm ? pip : ip;
         int width = 0;
         for (int i = 0; i < n; ++i) width = std::max(width, rp[i + 1] - rp[i]);
-        s->res = res::plan(width, nrhs, opts->precond, lptr, opts->team == 1 ? 1 : res::kMaxCtas);
+        s->res = res::plan(width, nrhs, opts->precond, lptr, one_cta ? 1 : res::kMaxCtas);
     }
     const size_t len = (size_t)n * nrhs;
     bool ok = upload(&s->lev_ptr, lptr);
@@ -2477,6 +2418,16 @@ struct kcfd_batch {
     int* cerr = nullptr;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // systems solved on chip (after the tiers in `order`), grouped by launch shape
+    struct Chip {
+        res::Plan plan;
+        int first, count;
+        cudaStream_t st;
+        cudaEvent_t ev;
+    };
+    std::vector<Chip> chip;
+    int nchip = 0;
+    int rep_huge = 0, rep_big = 0, rep_cl[kMaxClTiers] = {}, rep_ncl[kMaxClTiers] = {};  // by row count, chip ones included
 };
 
 namespace {
@@ -2485,6 +2436,10 @@ int free_batch(kcfd_batch* b) {
     if (b->side) cudaStreamDestroy(b->side);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
+    for (auto& c : b->chip) {
+        if (c.st) cudaStreamDestroy(c.st);
+        if (c.ev) cudaEventDestroy(c.ev);
+    }
     for (int t = 0; t < kcfd_batch::kMaxClTiers; ++t) {
         if (b->cst[t]) cudaStreamDestroy(b->cst[t]);
         if (b->cev[t]) cudaEventDestroy(b->cev[t]);
@@ -2659,15 +2614,42 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
         ncl_max[b->ntier++] = m;
     }
     const int nt = b->ntier;
+    // Tier by row count: a cluster tier, nt (one 512-thread CTA) or nt + 1 (one 256-thread CTA).
     auto tier = [&](int x) {
         for (int t = 0; t < nt; ++t)
             if (n[x] >= cand_rows[t]) return t;
         return (big_rows > 0 && n[x] >= big_rows) ? nt : nt + 1;
     };
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tier(x) < tier(y); });
-    b->nhuge = b->nbig = 0;
+    // With every tier option left to the library, FP64 systems that fit are solved on chip
+    // instead, on the fewest CTAs that hold them: a function of the system alone, so that its
+    // result is the same in any batch. Per SM and row that is also the fastest shape (Jacobi,
+    // 8 rows a thread: 3.4 ns per row and iteration; 4 rows 4.7, 1 row 15; in the tiers of
+    // this file 6-15 ns, the latter with every SM streaming).
+    std::vector<res::Plan> plan(nsys);
+    if (!mixed && b->o.cluster_rows == 0 && b->o.cluster_size == 0 && b->o.big_rows == 0 && b->o.lanes == 1) {
+        const int32_t* ip = indptr_host;
+        for (int s = 0; s < nsys; ip += n[s] + 1, ++s) {
+            int width = 0;
+            for (int i = 0; i < n[s]; ++i) width = std::max(width, ip[i + 1] - ip[i]);
+            plan[s] = res::plan_compact(n[s], width, b->o.precond);
+        }
+    }
+    auto on_chip = [&](int x) { return plan[x].ctas > 0; };
+    // one launch per shape, the largest clusters first
+    auto shape = [&](int x) { return plan[x].ctas * 16 + plan[x].rows_per_thread; };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        if (on_chip(x) != on_chip(y)) return on_chip(y);
+        return on_chip(x) ? shape(x) > shape(y) : tier(x) < tier(y);
+    });
     for (int s = 0; s < nsys; ++s) {
         const int t = tier(s);
+        b->rep_huge += t < nt ? 1 : 0;
+        b->rep_big += t == nt ? 1 : 0;
+        if (t < nt) b->rep_cl[t]++;
+        if (on_chip(s)) {
+            b->nchip++;
+            continue;
+        }
         if (t < nt) b->cl_n[t]++;
         b->nhuge += t < nt ? 1 : 0;
         b->nbig += t == nt ? 1 : 0;
@@ -2676,11 +2658,19 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
         b->cl_first[t] = first;
         first += b->cl_n[t];
         b->cl_ncl[t] = std::min(b->cl_n[t], ncl_max[t]);
+        b->rep_ncl[t] = std::min(b->rep_cl[t], ncl_max[t]);
+    }
+    for (int q = nsys - b->nchip; q < nsys; ++q) {
+        const int x = order[q];
+        if (b->chip.empty() || shape(x) != shape(order[q - 1])) b->chip.push_back({plan[x], q, 0, nullptr, nullptr});
+        auto& g = b->chip.back();
+        g.count++;
+        if (plan[x].width > g.plan.width) g.plan = plan[x];  // one width (and store size) per launch
     }
     int per_sm = 0, per_sm_big = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_ptr(mixed, b->o.precond, false), 256, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_big, batch_kernel_ptr(mixed, b->o.precond, true), 512, 0);
-    const int nsmall = nsys - b->nbig - b->nhuge;
+    const int nsmall = nsys - b->rep_big - b->rep_huge;
     b->grid = std::max(1, std::min(std::max(nsmall, 1), std::max(1, per_sm) * sms));
     b->grid_big = std::max(1, std::min(std::max(b->nbig, 1), std::max(1, per_sm_big) * sms));
     bool ok = cudaMalloc(&b->sys, nsys * sizeof(BatchSys)) == cudaSuccess &&
@@ -2705,6 +2695,9 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
              cudaStreamCreateWithFlags(&b->cst[t], cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&b->cev[t], cudaEventDisableTiming) == cudaSuccess;
     }
+    for (size_t g = 0; ok && g + 1 < b->chip.size(); ++g)  // the last group runs on the caller's stream
+        ok = cudaStreamCreateWithFlags(&b->chip[g].st, cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&b->chip[g].ev, cudaEventDisableTiming) == cudaSuccess;
     if (ok && b->nhuge > 0) ok = cudaMalloc(&b->cerr, sizeof(int)) == cudaSuccess;
     if (!ok) {
         free_batch(b);
@@ -2747,14 +2740,14 @@ int kcfd_batch_info(const kcfd_batch* b, int64_t* info) {
 
 int kcfd_batch_tiers(const kcfd_batch* b, int32_t* tiers) {
     KCFD_REQUIRE(b && tiers, "kcfd_batch_tiers: NULL argument");
-    tiers[0] = b->nhuge;
-    tiers[1] = b->nbig;
-    tiers[2] = b->nsys - b->nhuge - b->nbig;
+    tiers[0] = b->rep_huge;
+    tiers[1] = b->rep_big;
+    tiers[2] = b->nsys - b->rep_huge - b->rep_big;
     tiers[3] = 0;
     tiers[4] = 0;
     for (int t = 0; t < b->ntier; ++t) {
-        tiers[3] += b->cl_n[t] > 0 ? b->cl_ncl[t] : 0;
-        if (b->cl_n[t] > 0) tiers[4] = std::max(tiers[4], b->cl_size[t]);
+        tiers[3] += b->rep_cl[t] > 0 ? b->rep_ncl[t] : 0;
+        if (b->rep_cl[t] > 0) tiers[4] = std::max(tiers[4], b->cl_size[t]);
     }
     return KCFD_OK;
 }
@@ -2797,11 +2790,12 @@ int kcfd_batch_solve(kcfd_batch* b, const double* vals64, const double* rhs, dou
     for (int t = 0; t < b->ntier; ++t)
         if (b->cl_n[t] > 0) KCFD_CUDA(cudaMemsetAsync(b->cbar[t], 0, b->cl_ncl[t] * sizeof(unsigned int), st));
     if (b->nhuge > 0) KCFD_CUDA(cudaMemsetAsync(b->cerr, 0, sizeof(int), st));
-    B.nq = b->nsys;
+    B.nq = b->nsys - b->nchip;  // the on-chip kernel sets its systems up itself
     void* args[] = {&B};
-    const int pgrid = std::max(1, std::min(b->nsys, 4 * b->grid));
-    KCFD_CUDA(cudaLaunchKernel(B.mixed ? (void*)batch_prep_kernel<1> : (void*)batch_prep_kernel<0>, dim3(pgrid),
-                               dim3(256), args, 0, st));
+    const int pgrid = std::max(1, std::min(B.nq, 4 * b->grid));
+    if (B.nq > 0)
+        KCFD_CUDA(cudaLaunchKernel(B.mixed ? (void*)batch_prep_kernel<1> : (void*)batch_prep_kernel<0>, dim3(pgrid),
+                                   dim3(256), args, 0, st));
     // cluster tiers and the big tier on side streams, forked from and joined back into
     // the caller's; the cluster tiers are launched first (largest teams first) so that
     // their clusters find free SMs
@@ -2810,10 +2804,10 @@ int kcfd_batch_solve(kcfd_batch* b, const double* vals64, const double* rhs, dou
     Bb.nq = b->nbig;
     Bs.order = b->order + b->nhuge + b->nbig;
     Bs.queue = b->queue + 1;
-    Bs.nq = b->nsys - b->nhuge - b->nbig;
+    Bs.nq = b->nsys - b->nchip - b->nhuge - b->nbig;
     void* args_b[] = {&Bb};
     void* args_s[] = {&Bs};
-    if (b->nhuge > 0 || b->nbig > 0) KCFD_CUDA(cudaEventRecord(b->ev_fork, st));
+    if (b->nhuge > 0 || b->nbig > 0 || b->chip.size() > 1) KCFD_CUDA(cudaEventRecord(b->ev_fork, st));
     if (b->nbig > 0) KCFD_CUDA(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
     for (int t = 0; t < b->ntier; ++t) {
         if (b->cl_n[t] == 0) continue;
@@ -2838,6 +2832,14 @@ int kcfd_batch_solve(kcfd_batch* b, const double* vals64, const double* rhs, dou
                                    b->side));
     if (Bs.nq > 0)
         KCFD_CUDA(cudaLaunchKernel(batch_kernel_ptr(B.mixed, B.precond, false), dim3(b->grid), dim3(256), args_s, 0, st));
+    for (auto& g : b->chip) {
+        if (g.st) KCFD_CUDA(cudaStreamWaitEvent(g.st, b->ev_fork, 0));
+        KCFD_CUDA(res::batch(g.plan, B, g.first, g.count, g.st ? g.st : st));
+        if (g.st) {
+            KCFD_CUDA(cudaEventRecord(g.ev, g.st));
+            KCFD_CUDA(cudaStreamWaitEvent(st, g.ev, 0));
+        }
+    }
     if (b->nbig > 0) {
         KCFD_CUDA(cudaEventRecord(b->ev_join, b->side));
         KCFD_CUDA(cudaStreamWaitEvent(st, b->ev_join, 0));

@@ -35,7 +35,10 @@ class BatchSolver:
     cluster_rows (0: 16384) -- or one tier of cluster_size CTAs from cluster_rows rows
     (0: 131072); negative cluster_rows: none. Then at least big_rows rows (0: 16384,
     negative: none) by one 512-thread CTA; the rest by one 256-thread CTA. tiers()
-    reports the split (cluster_size: the largest team).
+    reports the split (cluster_size: the largest team). With all three left at 0 and
+    lanes 1, FP64 systems that fit the shared memory of a thread-block cluster (up to
+    32,768 rows) are solved on chip instead, whatever their tier, on the fewest CTAs
+    that hold them: a function of the system alone.
 
     restarts: with the scipy stopping rule, a system whose rho or omega breaks down
     restarts from its current iterate (rhat = r, p = r) up to this many times (0: it

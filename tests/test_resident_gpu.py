@@ -86,3 +86,37 @@ def test_many_levels_and_stop_rules(n):
     x = torch.zeros(n, dtype=torch.float64, device="cuda")
     it, rr, st = s.solve(d, torch.from_numpy(b).cuda(), x)
     assert int(st[0]) == _lib.MAXITER and int(it[0]) == 3
+
+
+@pytest.mark.parametrize("prec", ["none", "jacobi"])
+def test_batch_on_chip(prec):
+    """A batch around the steps of the on-chip shapes (CTAs, rows per thread) and one system past the largest:
+    against the grid kernel, and bitwise the same alone."""
+    import torch
+    from kcfd.batch import BatchSolver
+    from kcfd.solver import DeviceCSR, Solver
+    sizes = [1, 40, 256, 257, 1025, 2047, 2048, 2049, 3073, 4097, 10241, 12289, 20481, 32768, 32769]
+    mats = [system(n, seed=n, nonsym=0.2) for n in sizes]
+    rng = np.random.default_rng(7)
+    rhs = [rng.standard_normal(n) for n in sizes]
+    pats = [(A.indptr.astype(np.int32), A.indices.astype(np.int32)) for A in mats]
+
+    def solve(ids):
+        B = BatchSolver([pats[k] for k in ids], mode="fp64", precond=prec, rtol=1e-12, maxiter=5000)
+        x = torch.zeros(B.n_total, dtype=torch.float64, device="cuda")
+        vals = torch.from_numpy(np.concatenate([mats[k].data for k in ids])).cuda()
+        _, rr, st = B.solve(vals, B.pack([rhs[k] for k in ids]), x)
+        assert st.tolist() == [0] * len(ids) and float(rr.max()) < 1e-12
+        return B.unpack(x)
+
+    xs = solve(range(len(sizes)))
+    for k, n in enumerate(sizes):
+        d = DeviceCSR.from_scipy(mats[k])
+        s = Solver(d, precond=prec, rtol=1e-12, maxiter=5000, team=2)
+        s.setup(d)
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        s.solve(d, torch.from_numpy(rhs[k]).cuda(), x)
+        ref = x.cpu().numpy()
+        assert np.linalg.norm(xs[k] - ref) <= 1e-9 * np.linalg.norm(ref)
+    for k in (3, 9, 12):
+        np.testing.assert_array_equal(solve([k])[0], xs[k])
