@@ -211,7 +211,11 @@ typedef struct {
                             replacement against the FP64 matrix -- for well
                             conditioned systems, so only when asked for). Auto:
                             1 for n*nrhs <= 1024, 2 up to 40000 and for MIXED,
-                            else 3.                                              
+                            else 3; with 1 or 2 chosen so (lanes and block 0), an
+                            FP64 system that fits the shared memory of a
+                            thread-block cluster is solved there (as is one that
+                            fits a single CTA with team 1, lanes <= 1 and block
+                            0 or 256).
                             KCFD_ENGINE_EAGER=1 in the environment at creation
                             launches the engine's kernels from a host loop
                             instead (for profilers; same results);
@@ -240,6 +244,10 @@ typedef struct {
  * (FP64 arithmetic). Inside a stream capture an AMG handle does not solve (the
  * engine's graph is not nested): the call returns KCFD_BAD_INPUT.                 */
 
+/* Greedy colouring of the symmetrised matrix graph, rows in index order (host only): the
+ * row levels of a multicolour ILU(0) for a matrix that comes without a mesh. Two coupled
+ * rows never share a colour.                                                         */
+int kcfd_row_colouring(int32_t n, const int32_t* indptr_host, const int32_t* indices_host, int32_t* colour);
 /* ILU(0) ordering: level_of_row_host gives each row's level (e.g. the mesh's cell
  * colouring, or natural-order dependency levels); NULL -> natural-order levels.
  * Coupled rows must lie on different levels. With ILU(0) the handle solves the

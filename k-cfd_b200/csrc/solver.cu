@@ -1925,6 +1925,19 @@ void kcfd_graph_destroy(kcfd_graph* g) {
     delete g;
 }
 
+int kcfd_row_colouring(int32_t n, const int32_t* indptr, const int32_t* indices, int32_t* colour) {
+    KCFD_REQUIRE(indptr && indices && colour && n > 0 && indptr[0] == 0, "kcfd_row_colouring: bad pattern");
+    for (int i = 0; i < n; ++i) {
+        KCFD_REQUIRE(indptr[i + 1] >= indptr[i], "kcfd_row_colouring: indptr not monotone at row %d", i);
+        for (int k = indptr[i]; k < indptr[i + 1]; ++k)
+            KCFD_REQUIRE(indices[k] >= 0 && indices[k] < n, "kcfd_row_colouring: column index out of range at %d", k);
+    }
+    const std::vector<int> c = distance_colouring(n, std::vector<int>(indptr, indptr + n + 1),
+                                                  std::vector<int>(indices, indices + indptr[n]), 1);
+    std::copy(c.begin(), c.end(), colour);
+    return KCFD_OK;
+}
+
 int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, const int32_t* level_of_row_host,
                        kcfd_solver** out) {
     KCFD_REQUIRE(A && opts && out, "kcfd_solver_create: NULL argument");
@@ -2192,7 +2205,7 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     }
     const size_t len = (size_t)n * nrhs;
     bool ok = upload(&s->lev_ptr, lptr);
-    ok = ok && cudaMalloc(&s->work, 9 * len * vsz) == cudaSuccess;
+    if (s->res.ctas == 0) ok = ok && cudaMalloc(&s->work, 9 * len * vsz) == cudaSuccess;  // on chip: no scratch
     if (mixed) ok = ok && cudaMalloc(&s->r64, len * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&s->bar, 2 * sizeof(unsigned)) == cudaSuccess;
     ok = ok && cudaMalloc(&s->err, sizeof(int)) == cudaSuccess;

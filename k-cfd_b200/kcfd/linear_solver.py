@@ -18,7 +18,10 @@ device failure raises instead of falling back to the CPU. Semantics kept:
     agreement is at the solution level; max_levels and max_coarse are honoured, the
     coarsest level being at most 256 rows).
   * method='direct': the device has no sparse LU; BiCGSTAB + ILU(0) to a relative
-    residual of 1e-12 stands in for spsolve (documented difference).
+    residual of 1e-12 stands in for spsolve (documented difference). A matrix without
+    ILU levels of its own is coloured first: natural-order levels are some hundred
+    short dependent steps per sweep (5,000 triangles, whole call: 84 ms against 7.4 ms coloured);
+    they are the second try where the coloured factor does not converge.
 system may be the reference's FVMSystem (anything with .to_sparse() and .rhs), a
 kcfd FVMSystem, or a device-assembled kcfd DeviceSystem.
 """
@@ -89,6 +92,15 @@ def _as_device(system):
     return DeviceCSR.from_scipy(A), b, None
 
 
+def _colour_levels(d):
+    """Greedy row colouring of the matrix graph, as ILU(0) levels (kcfd_row_colouring)."""
+    ip, ix = d.indptr.cpu().numpy(), d.indices.cpu().numpy()
+    lev = np.empty(d.n, dtype=np.int32)
+    _lib.check(_lib.lib().kcfd_row_colouring(d.n, ip.ctypes.data, ix.ctypes.data, lev.ctypes.data),
+               "kcfd_row_colouring")
+    return lev
+
+
 def solve_linear_system(system, x0=None, method="direct", tol=1e-8, maxiter=1000, backend="auto",
                         preconditioner="none", **precond_kwargs):
     if backend not in ("auto", "b200", "gpu"):
@@ -116,11 +128,17 @@ def solve_linear_system(system, x0=None, method="direct", tol=1e-8, maxiter=1000
     if prec == "amg":
         amg_kw = {"amg_max_levels": int(precond_kwargs.pop("max_levels", 0)),
                   "amg_coarse_max": min(int(precond_kwargs.pop("max_coarse", 0)), 256)}
-    s = Solver(d, precond=prec, stop=_lib.STOP_SCIPY, maxiter=its, rtol=rtol_eff, atol=atol, levels=levels,
-               fill_level=fill, **amg_kw)
-    s.setup(d)
-    it, rr, st = s.solve(d, b, x)
-    status = int(st[0])
+    tries = [levels] if method != "direct" or levels is not None else [_colour_levels(d), None]
+    x_start = x.clone() if len(tries) > 1 else x
+    for lev in tries:
+        s = Solver(d, precond=prec, stop=_lib.STOP_SCIPY, maxiter=its, rtol=rtol_eff, atol=atol, levels=lev,
+                   fill_level=fill, **amg_kw)
+        s.setup(d)
+        it, rr, st = s.solve(d, b, x)
+        status = int(st[0])
+        if status == _lib.OK or lev is tries[-1]:
+            break
+        x.copy_(x_start)
     if status == _lib.MAXITER and method == "bicgstab":
         print(f"[bicgstab] 수렴 실패: {int(it[0])} 반복 후 중단")
     elif status not in (_lib.OK, _lib.MAXITER, _lib.BREAKDOWN):

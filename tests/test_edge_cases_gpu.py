@@ -120,3 +120,19 @@ def test_batch_single_system_and_both_tiers(torch_cuda):
         assert list(st.cpu().numpy()) == [0] * len(pick)
         for xs, k in zip(bs.unpack(x), pick):
             assert np.linalg.norm(rhs[k] - mats[k] @ xs) / np.linalg.norm(rhs[k]) < 2e-10
+
+
+@pytest.mark.parametrize("n", [1, 7, 900])
+def test_direct_colours_a_host_matrix(n):
+    """method='direct' on a host CSR: the multicolour ILU(0) (a non-symmetric, convection-like matrix) solves to
+    1e-12, and caller-given levels are used as they are."""
+    from kcfd.fvm_operators import FVMSystem
+    from kcfd.linear_solver import solve_linear_system
+    rng = np.random.default_rng(n)
+    A = sparse.diags([-rng.uniform(0.1, 1.9, max(n - 1, 0)), np.full(n, 3.0), -rng.uniform(0.1, 0.9, max(n - 1, 0))],
+                     [-1, 0, 1], shape=(n, n)).tocsr()
+    s = FVMSystem.from_csr(A, rng.standard_normal(n))
+    x = solve_linear_system(s)
+    assert np.linalg.norm(A @ x - s.rhs) <= 2e-12 * np.linalg.norm(s.rhs)
+    y = solve_linear_system(s, levels=np.arange(n, dtype=np.int32))
+    assert np.linalg.norm(A @ y - s.rhs) <= 2e-12 * np.linalg.norm(s.rhs)

@@ -67,3 +67,21 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     with pytest.raises(RuntimeError, match="nvcc not found"):
         _lib.lib()
     assert _lib._lib is None
+
+
+def test_row_colouring_separates_coupled_rows():
+    """kcfd_row_colouring (host only): no two coupled rows share a colour, whichever side stores the entry."""
+    import numpy as np
+    from scipy import sparse
+    from kcfd import _lib
+    rng = np.random.default_rng(1)
+    for n in (1, 2, 50, 400):
+        A = (sparse.random(n, n, 0.02, random_state=rng, format="csr") + sparse.eye(n)).tocsr()
+        ip, ix = A.indptr.astype(np.int32), A.indices.astype(np.int32)
+        c = np.full(n, -1, np.int32)
+        assert _lib.lib().kcfd_row_colouring(n, ip.ctypes.data, ix.ctypes.data, c.ctypes.data) == _lib.OK
+        r = np.repeat(np.arange(n), np.diff(ip))
+        assert c.min() >= 0 and (c[r] != c[ix])[r != ix].all()
+    bad = np.array([5], np.int32)
+    one = np.array([0, 1], np.int32)
+    assert _lib.lib().kcfd_row_colouring(1, one.ctypes.data, bad.ctypes.data, c.ctypes.data) == _lib.BAD_INPUT
