@@ -10,14 +10,16 @@
 //   volume fraction       models/two_fluid.py:727-783
 //   phase energy          models/two_fluid.py:412-518
 //   boundary refresh      models/two_fluid.py:224-250; mass flux core/interpolation.py:163-182
-// Face kernels run one launch per face colour (no two faces of a colour share a
-// cell), so every scatter is free of write conflicts and of atomics; per-element
-// arithmetic follows the reference's expression order.
+// Face loops run by cell, together with the cell terms that go into the same sums
+// (by_cell.cuh); on a mesh without cell lists, one launch per face colour (no two faces
+// of a colour share a cell). Either way no scatter has write conflicts or atomics;
+// per-element arithmetic follows the reference's expression order.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
 
+#include "by_cell.cuh"
 #include "kcfd_common.h"
 
 namespace kcfd {
@@ -404,6 +406,159 @@ __global__ void k_strided_copy(int n, int nc_copy, const double* __restrict__ sr
         for (int c = 0; c < nc_copy; ++c) dst[(int64_t)i * ds + dof + c] = src[(int64_t)i * ss + so + c];
 }
 
+// Momentum cell terms (k_mom_cells_tf) and the pressure force (k_mom_pressure).
+struct MomentumOp {
+    int nd, comp0, nc;
+    kcfd_tf_params_t P;
+    double rho;
+    const double *alpha, *p, *K, *Uo, *old;
+    double *v, *diag, *rhs;
+    static constexpr bool kOff = false;
+    struct Acc {
+        double s[3], a, p;
+    };
+    struct Data {
+        double p, A, n[3];
+    };
+    __device__ Acc begin(const kcfd_dmesh_t&, int i) const { return {{0.0, 0.0, 0.0}, __ldg(alpha + i), __ldg(p + i)}; }
+    __device__ Data load(const kcfd_dmesh_t& m, int, const CellFace& c, const Acc&) const {
+        Data d{__ldg(p + c.other), __ldg(m.area + c.f), {0.0, 0.0, 0.0}};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (k < nc) d.n[k] = __ldg(m.normal + c.f * nd + comp0 + k);
+        return d;
+    }
+    __device__ double apply(const CellFace& c, const Data& d, Acc& a) const {
+        const double pf = 0.5 * (a.p + d.p), s = c.own ? -a.a : a.a;  // the own p on a boundary face
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a.s[k] += s * pf * d.n[k] * d.A;
+        return 0.0;
+    }
+    __device__ void end(const kcfd_dmesh_t& m, int i, const Acc& a) const {
+        const double V = __ldg(m.volume + i), kv = K[i] * V;
+        const double c = old ? a.a * rho * V / P.dt : 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (k >= nc) break;
+            double r = rhs[i * nc + k];
+            if (old) r += c * old[i * nd + comp0 + k];
+            r += kv * Uo[i * nd + comp0 + k];
+            r += a.a * rho * P.g[comp0 + k] * V;
+            rhs[i * nc + k] = r + a.s[k];
+        }
+        const int s = __ldg(m.diag_slot + i);
+        v[s] = (v[s] + c) + kv;
+        diag[i] = (diag[i] + c) + kv;
+    }
+};
+
+// Two-phase pressure correction (k_pp_int_tf, k_pp_bnd_tf, k_pin).
+struct PressureOp {
+    kcfd_tf_params_t P;
+    const double *al, *ag, *apl, *apg, *mfl, *mfg;
+    double *v, *diag, *rhs;
+    static constexpr bool kOff = true;
+    struct Acc {
+        double s[2], al, ag, apl, apg, V;
+    };
+    struct Data {
+        double d, A, fl, fg, al, ag, apl, apg, V;
+    };
+    __device__ Acc begin(const kcfd_dmesh_t& m, int i) const {
+        return {{0.0, 0.0}, __ldg(al + i), __ldg(ag + i), __ldg(apl + i), __ldg(apg + i), __ldg(m.volume + i)};
+    }
+    __device__ Data load(const kcfd_dmesh_t& m, int, const CellFace& c, const Acc&) const {
+        return {__ldg(m.dlen + c.f), __ldg(m.area + c.f), __ldg(mfl + c.f), __ldg(mfg + c.f), __ldg(al + c.other),
+                __ldg(ag + c.other), __ldg(apl + c.other), __ldg(apg + c.other), __ldg(m.volume + c.other)};
+    }
+    __device__ double apply(const CellFace& c, const Data& d, Acc& a) const {
+        if (c.in && d.d < 1e-30) return 0.0;
+        const double tot = d.fl * (c.own ? a.al : d.al) + d.fg * (c.own ? a.ag : d.ag);
+        a.s[1] += c.own ? -tot : tot;
+        if (!c.in) return 0.0;
+        const double al_f = 0.5 * (a.al + d.al), ag_f = 0.5 * (a.ag + d.ag);
+        const double apl_f = 0.5 * (a.apl + d.apl), apg_f = 0.5 * (a.apg + d.apg), vol_f = 0.5 * (a.V + d.V);
+        const double cl = P.rho_l * al_f * vol_f / fmax(apl_f, 1e-30);
+        const double cg = P.rho_g * ag_f * vol_f / fmax(apg_f, 1e-30);
+        const double k = (cl + cg) * d.A / d.d;
+        a.s[0] += k;
+        return -k;
+    }
+    __device__ void end(const kcfd_dmesh_t& m, int i, const Acc& a) const {
+        const double pin = i == 0 ? 1e10 : 0.0;
+        const int s = __ldg(m.diag_slot + i);
+        v[s] = (v[s] + a.s[0]) + pin;
+        diag[i] = (diag[i] + a.s[0]) + pin;
+        rhs[i] += a.s[1];
+    }
+};
+
+// Difference gradient of p' (k_grad_diff) and the correction (k_correct_tf).
+template <int D>
+struct CorrectOp {
+    double alpha_p;
+    const double *pp, *al, *ag, *apl, *apg;
+    double *grad, *Ul, *Ug, *p;
+    static constexpr bool kOff = false;
+    struct Acc {
+        double s[D], pp;
+    };
+    struct Data {
+        double pp, A, n[D];
+    };
+    __device__ Acc begin(const kcfd_dmesh_t&, int i) const {
+        Acc a;
+        a.pp = __ldg(pp + i);
+#pragma unroll
+        for (int k = 0; k < D; ++k) a.s[k] = 0.0;
+        return a;
+    }
+    __device__ Data load(const kcfd_dmesh_t& m, int, const CellFace& c, const Acc&) const {
+        Data d;
+        d.pp = __ldg(pp + c.other);
+        d.A = __ldg(m.area + c.f);
+#pragma unroll
+        for (int k = 0; k < D; ++k) d.n[k] = __ldg(m.normal + c.f * D + k);
+        return d;
+    }
+    __device__ double apply(const CellFace&, const Data& d, Acc& a) const {
+        // pp[neighbour] - pp[owner] is added on the owner side; on the neighbour side the
+        // same product is negated twice; 0 on a boundary face
+        const double dp = d.pp - a.pp;
+#pragma unroll
+        for (int k = 0; k < D; ++k) a.s[k] += dp * d.n[k] * d.A;
+        return 0.0;
+    }
+    __device__ void end(const kcfd_dmesh_t& m, int i, const Acc& a) const {
+        const double V = __ldg(m.volume + i);
+        p[i] = p[i] + alpha_p * a.pp;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            grad[i * D + k] = a.s[k];
+            double g = a.s[k];
+            if (V > 1e-30) g = g / V;
+            const double cl = -al[i] * V / fmax(apl[i], 1e-20) * g;
+            const double cg = -ag[i] * V / fmax(apg[i], 1e-20) * g;
+            Ul[i * D + k] += alpha_p * cl;
+            Ug[i * D + k] += alpha_p * cg;
+        }
+    }
+};
+
+// Wall heat flux on the boundary faces of heated patches (k_wall_flux).
+struct WallFluxOp {
+    const int8_t* qmask;
+    const double *q, *aw;
+    double* rhs;
+    using Acc = double;
+    __device__ Acc begin(const kcfd_dmesh_t&, int i) const { return rhs[i]; }
+    __device__ void face(const kcfd_dmesh_t& m, int i, int f, Acc& a) const {
+        const int bi = f - m.n_internal;
+        if (qmask[bi]) a += q[bi] * __ldg(m.area + f) * aw[i];
+    }
+    __device__ void end(const kcfd_dmesh_t&, int i, const Acc& a) const { rhs[i] = a; }
+};
+
 int chk(const kcfd_dmesh_t* m) {
     KCFD_REQUIRE(m && m->owner && m->color_ptr && m->diag_slot, "kcfd_tf: NULL mesh descriptor");
     KCFD_REQUIRE(m->ndim == 2 || m->ndim == 3, "kcfd_tf: ndim must be 2 or 3");
@@ -491,6 +646,11 @@ int kcfd_tf_momentum_sources(const kcfd_dmesh_t* m, const kcfd_tf_params_t* P, i
     KCFD_REQUIRE(P && alpha && p && K && U_other && vals && diag && rhs, "kcfd_tf_momentum_sources: NULL argument");
     KCFD_REQUIRE(comp0 >= 0 && nc >= 1 && comp0 + nc <= m->ndim, "kcfd_tf_momentum_sources: bad components");
     cudaStream_t st = (cudaStream_t)stream;
+    if (has_cell_lists(m)) {
+        by_cell(m, MomentumOp{m->ndim, comp0, nc, *P, rho, alpha, p, K, U_other, U_old, vals, diag, rhs}, st);
+        KCFD_CUDA(cudaGetLastError());
+        return KCFD_OK;
+    }
     k_mom_cells_tf<<<nblk(m->n_cells), kT, 0, st>>>(m->n_cells, m->ndim, comp0, nc, *P, rho, m->diag_slot, m->volume,
                                                     alpha, K, U_other, U_old, vals, diag, rhs);
     auto pf = [&](int f0, int f1, int nb) { k_mom_pressure<<<nb, kT, 0, st>>>(*m, f0, f1, comp0, nc, alpha, p, rhs); };
@@ -506,7 +666,8 @@ int kcfd_tf_boundary(const kcfd_dmesh_t* m, const int8_t* btype, const double* b
     KCFD_REQUIRE(btype && bval && bgrad && gamma && mf && vals && diag && rhs && nc >= 1 && nc <= 3,
                  "kcfd_tf_boundary: bad arguments");
     cudaStream_t st = (cudaStream_t)stream;
-    tf_colours(m, false, [&](int f0, int f1, int nb) {
+    if (has_cell_lists(m)) by_boundary_cell(m, BoundaryOp{btype, bval, bgrad, nc, gamma, mf, vals, diag, rhs}, st);
+    else tf_colours(m, false, [&](int f0, int f1, int nb) {
         k_bc_tf<<<nb, kT, 0, st>>>(*m, f0, f1, btype, bval, bgrad, nc, gamma, mf, vals, diag, rhs);
     });
     KCFD_CUDA(cudaGetLastError());
@@ -538,6 +699,11 @@ int kcfd_tf_pressure_assemble(const kcfd_dmesh_t* m, const kcfd_tf_params_t* P, 
     KCFD_REQUIRE(P && alpha_l && alpha_g && aP_l && aP_g && mf_l && mf_g && vals && diag && rhs,
                  "kcfd_tf_pressure_assemble: NULL argument");
     cudaStream_t st = (cudaStream_t)stream;
+    if (has_cell_lists(m)) {
+        by_cell(m, PressureOp{*P, alpha_l, alpha_g, aP_l, aP_g, mf_l, mf_g, vals, diag, rhs}, st);
+        KCFD_CUDA(cudaGetLastError());
+        return KCFD_OK;
+    }
     tf_colours(m, true, [&](int f0, int f1, int nb) {
         k_pp_int_tf<<<nb, kT, 0, st>>>(*m, f0, f1, *P, alpha_l, alpha_g, aP_l, aP_g, mf_l, mf_g, vals, diag, rhs);
     });
@@ -555,6 +721,14 @@ int kcfd_tf_correct(const kcfd_dmesh_t* m, double alpha_p, const double* pp, con
     if (int e = chk(m)) return e;
     KCFD_REQUIRE(pp && alpha_l && alpha_g && aP_l && aP_g && grad && U_l && U_g && p, "kcfd_tf_correct: NULL argument");
     cudaStream_t st = (cudaStream_t)stream;
+    if (has_cell_lists(m)) {
+        if (m->ndim == 2)
+            by_cell(m, CorrectOp<2>{alpha_p, pp, alpha_l, alpha_g, aP_l, aP_g, grad, U_l, U_g, p}, st);
+        else
+            by_cell(m, CorrectOp<3>{alpha_p, pp, alpha_l, alpha_g, aP_l, aP_g, grad, U_l, U_g, p}, st);
+        KCFD_CUDA(cudaGetLastError());
+        return KCFD_OK;
+    }
     KCFD_CUDA(cudaMemsetAsync(grad, 0, sizeof(double) * (size_t)m->n_cells * m->ndim, st));
     tf_colours(m, true, [&](int f0, int f1, int nb) { k_grad_diff<<<nb, kT, 0, st>>>(*m, f0, f1, pp, grad); });
     k_correct_tf<<<nblk(m->n_cells), kT, 0, st>>>(m->n_cells, m->ndim, alpha_p, m->volume, pp, alpha_l, alpha_g, aP_l,
@@ -581,7 +755,8 @@ int kcfd_tf_energy_sources(const kcfd_dmesh_t* m, const kcfd_tf_params_t* P, dou
     cudaStream_t st = (cudaStream_t)stream;
     k_energy_cells<<<nblk(m->n_cells), kT, 0, st>>>(m->n_cells, *P, rho, cp, m->diag_slot, m->volume, alpha, T_old,
                                                     T_other, hiaiV, dot_m, dm_sign, vals, diag, rhs);
-    tf_colours(m, false, [&](int f0, int f1, int nb) {
+    if (has_cell_lists(m)) by_boundary_cell(m, WallFluxOp{qmask, q_b, alpha_wall, rhs}, st);
+    else tf_colours(m, false, [&](int f0, int f1, int nb) {
         k_wall_flux<<<nb, kT, 0, st>>>(*m, f0, f1, qmask, q_b, alpha_wall, rhs);
     });
     KCFD_CUDA(cudaGetLastError());
