@@ -211,11 +211,13 @@ typedef struct {
                             replacement against the FP64 matrix -- for well
                             conditioned systems, so only when asked for). Auto:
                             1 for n*nrhs <= 1024, 2 up to 40000 and for MIXED,
-                            else 3; with 1 or 2 chosen so (lanes and block 0), an
-                            FP64 system that fits the shared memory of a
-                            thread-block cluster is solved there (as is one that
-                            fits a single CTA with team 1, lanes <= 1 and block
-                            0 or 256).
+                            else 3. With the choice left so (lanes and block 0)
+                            a FP64 BiCGSTAB solve with Jacobi, ILU or no
+                            preconditioner whose system fits on chip runs there
+                            instead: in the shared memory and registers of a
+                            thread-block cluster, or of one CTA per SM (a
+                            cooperative launch). So does one that fits a single
+                            CTA with team 1, lanes <= 1 and block 0 or 256.
                             KCFD_ENGINE_EAGER=1 in the environment at creation
                             launches the engine's kernels from a host loop
                             instead (for profilers; same results);

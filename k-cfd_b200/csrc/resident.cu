@@ -13,14 +13,32 @@ template <int NRHS, int PREC, int R>
 __global__ void __launch_bounds__(kBlock, 1) k_resident(SolveArgs a, int width) {
     extern __shared__ __align__(16) char store[];
     __shared__ Shared sh;
-    Team tm;
+    ClusterTeam tm;
     int id;
     cluster_ids(tm.rank, tm.size, id);
     tm.sh = &sh;
     tm.budget = a.ctl.budget;
     tm.init();
     solve_on_chip<NRHS, PREC, R>(tm, a, width, store);
-    tm.sync();  // no CTA leaves while another may still gather from it
+    tm.finish();
+}
+
+// One CTA per SM, for systems beyond a cluster. scratch: the gathered vector, then the
+// partials of the reductions.
+template <int NRHS, int PREC, int R>
+__global__ void __launch_bounds__(kBlock, 1) k_resident_grid(SolveArgs a, int width, double* scratch) {
+    extern __shared__ __align__(16) char store[];
+    __shared__ Shared sh;
+    GridTeam tm;
+    tm.rank = blockIdx.x;
+    tm.size = gridDim.x;
+    tm.sh = &sh;
+    tm.budget = a.ctl.budget;
+    tm.count = a.ctl.bar;
+    tm.err = a.ctl.err;
+    tm.part = scratch + (size_t)(a.n + 1) * NRHS;
+    tm.init();
+    solve_on_chip<NRHS, PREC, R>(tm, a, width, store, scratch);
 }
 
 // Systems B.order[first + cluster index]: independent solves, one cluster each, scheduled by
@@ -29,7 +47,7 @@ template <int PREC, int R>
 __global__ void __launch_bounds__(kBlock, 1) k_resident_batch(BatchArgs B, int first, int width, long long budget) {
     extern __shared__ __align__(16) char store[];
     __shared__ Shared sh;
-    Team tm;
+    ClusterTeam tm;
     int id;
     cluster_ids(tm.rank, tm.size, id);
     tm.sh = &sh;
@@ -38,7 +56,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_resident_batch(BatchArgs B, int f
     SolveArgs a = batch_args<double>(B, B.order[first + id]);
     a.dinv = nullptr;
     solve_on_chip<1, PREC, R>(tm, a, width, store);
-    tm.sync();
+    tm.finish();
 }
 
 namespace {
@@ -55,14 +73,18 @@ bool dispatch(int nrhs, int precond, int r, F f) {
 #define KC_RES_P(N, RR) KC_RES(N, 0, RR) KC_RES(N, 1, RR) KC_RES(N, 2, RR)
     KC_RES_P(1, 1) KC_RES_P(1, 2) KC_RES_P(1, 3) KC_RES_P(1, 4) KC_RES_P(1, 6) KC_RES_P(1, 8)
     KC_RES_P(2, 1) KC_RES_P(2, 2) KC_RES_P(2, 4)
-    KC_RES_P(3, 1) KC_RES_P(3, 2)
+    KC_RES_P(3, 1) KC_RES_P(3, 2) KC_RES_P(3, 3)
 #undef KC_RES_P
 #undef KC_RES
     return false;
 }
 
-void* kernel_of(int nrhs, int precond, int r) {  // nrhs 0: the batched kernel
+void* kernel_of(int nrhs, int precond, int r) {  // nrhs 0: the batched kernel; nrhs + 4: the grid's
     void* k = nullptr;
+    if (nrhs > 4) {
+        dispatch(nrhs - 4, precond, r, [&](auto n, auto p, auto rr) { k = (void*)k_resident_grid<n(), p(), rr()>; });
+        return k;
+    }
     if (nrhs == 0) {
         dispatch(1, precond, r, [&](auto, auto p, auto rr) {
             if constexpr (p() != KCFD_PREC_ILU0) k = (void*)k_resident_batch<p(), rr()>;
@@ -99,7 +121,7 @@ struct Limits {
 Limits limits(int nrhs, int precond, int r) {
     constexpr int kDevices = 64;
     static std::mutex mu;
-    static Limits known[kDevices][4][3][9];
+    static Limits known[kDevices][8][3][9];
     int dev = 0;
     void* f = kernel_of(nrhs, precond, r);
     if (!f || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return Limits();
@@ -117,6 +139,12 @@ Limits limits(int nrhs, int precond, int r) {
     }
     Plan p;
     p.smem = optin - (int)fa.sharedSizeBytes;
+    if (nrhs > 4) {
+        if (cudaDeviceGetAttribute(&L.ctas, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return Limits();
+        L.ctas = std::min(L.ctas, kMaxGrid);
+        L.smem = p.smem;
+        return L;
+    }
     for (p.ctas = kMaxCtas; p.ctas > 1; p.ctas /= 2) {
         int m = 0;
         cudaLaunchAttribute at[1];
@@ -134,16 +162,19 @@ Limits limits(int nrhs, int precond, int r) {
 Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max_ctas) {
     const int nlev = (int)lev.size() - 1;
     if (width < 1 || width > 64 || nlev > 4096) return Plan();
+    auto rows_on = [&](int ctas) {
+        int64_t rows = 0;
+        for (int l = 0; l < nlev; ++l) rows += (lev[l + 1] - lev[l] + ctas - 1) / ctas;
+        return rows;
+    };
     // the fewest rows per thread first: a thread's rows are done one after another
     for (int r = 1; r <= 8; ++r) {
         const Limits L = limits(nrhs, precond, r);
         size_t bytes = SIZE_MAX;
-        dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr()>::bytes(width, nlev); });
+        dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr(), false>::bytes(width, nlev); });
         if (L.smem == 0 || bytes > (size_t)L.smem) continue;
         for (int c = 1; c <= std::min(max_ctas, L.ctas); ++c) {
-            int64_t rows = 0;
-            for (int l = 0; l < nlev; ++l) rows += (lev[l + 1] - lev[l] + c - 1) / c;
-            if (rows > kBlock * r) continue;
+            if (rows_on(c) > kBlock * r) continue;
             Plan p;
             p.ctas = c;
             p.rows_per_thread = r;
@@ -151,6 +182,21 @@ Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max
             p.smem = (int)bytes;
             return p;
         }
+    }
+    // beyond a cluster: one CTA per SM
+    for (int r = 1; r <= 8 && max_ctas > 1; ++r) {
+        const Limits L = limits(nrhs + 4, precond, r);
+        size_t bytes = SIZE_MAX;
+        dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr(), true>::bytes(width, nlev); });
+        if (L.smem == 0 || bytes > (size_t)L.smem || rows_on(L.ctas) > kBlock * r) continue;
+        Plan p;
+        p.ctas = L.ctas;
+        p.grid = true;
+        p.rows_per_thread = r;
+        p.width = width;
+        p.smem = (int)bytes;
+        p.scratch = (size_t)(lev[nlev] + 1) * nrhs + (size_t)2 * kMaxQ * L.ctas;
+        return p;
     }
     return Plan();
 }
@@ -184,9 +230,17 @@ cudaError_t batch(const Plan& p, const BatchArgs& B, int first, int count, cudaS
     return cudaLaunchKernelExC(&cfg, kernel_of(0, B.precond, p.rows_per_thread), ptrs);
 }
 
-cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, cudaStream_t st) {
+cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, double* scratch, cudaStream_t st) {
     SolveArgs args = a;
     int width = p.width;
+    if (p.grid) {
+        void* ptrs[] = {&args, &width, &scratch};
+        cudaError_t e = cudaMemsetAsync(a.ctl.bar, 0, sizeof(unsigned), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a.ctl.err, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+        return cudaLaunchCooperativeKernel(kernel_of(nrhs + 4, precond, p.rows_per_thread), dim3(p.ctas), dim3(kBlock), ptrs,
+                                           p.smem, st);
+    }
     void* ptrs[] = {&args, &width};
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = config(p, st, at);

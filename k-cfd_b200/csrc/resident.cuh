@@ -27,10 +27,19 @@
 //    which broadcasts what the vector phases need.
 // The hardware keeps the CTAs of a cluster resident together; the waits on an mbarrier are
 // bounded all the same (status KCFD_TIMEOUT).
+//
+// Larger systems take the same iteration on one cooperative launch with a CTA per SM
+// (GridTeam): matrix and vectors on chip as above, the gathered vector in global memory (it
+// stays in L2), a counter there for the barriers (2,450 cycles, whatever the CTA count) and
+// the CTAs' partials beside it (3,400 to 4,100 cycles a reduction). As kernels of a graph
+// loop the same steps cost 3.8 us each beyond their launch, most of it in the reductions'
+// last-block hand-over: 45 us per ILU(0) iteration on 48^3 hexes, where this takes 22.5
+// (Jacobi 30 and 11.5, three right-hand sides 58 and 19).
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "kcfd_common.h"
 #include "resident.h"
@@ -42,6 +51,7 @@ namespace res {
 constexpr int kBlock = 256;
 constexpr int kWarps = kBlock / 32;
 constexpr int kMaxQ = 9;   // values per reduction (three per right-hand side)
+constexpr int kMaxGrid = 160;  // CTAs of the grid form
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -82,15 +92,35 @@ enum { kDone = 1, kSconv = 2, kRestart = 4, kZero = 8 };
 struct Shared {
     uint64_t bar[2];                     // arrivals of the CTAs' partials, alternating
     double warp[kMaxQ * kWarps];         // partials of this CTA's warps
-    double part[2][kMaxQ * kMaxCtas];    // partials of the CTAs, 0 for absent ones
+    double part[2][kMaxQ * kMaxCtas];    // partials of a cluster's CTAs, 0 for absent ones
+    double total[kMaxQ];                 // totals over the grid
     double al[3], om[3], be[3];          // alpha, omega, beta of each right-hand side
     int flags[3];
     int fail;                            // a wait expired
     int status, iters;                   // of right-hand side 0, after a pass
 };
 
+// Sums over each warp of its threads' Q values, into sh->warp; a block barrier follows.
+template <int Q>
+__device__ __forceinline__ void warp_sums(double (&v)[Q], Shared* sh) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        double y[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) y[q] = __shfl_xor_sync(0xffffffffu, v[q], o);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) v[q] += y[q];
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) sh->warp[q * kWarps + wid] = v[q];
+    }
+}
+
 // The CTAs of one cluster; `uses` counts reductions (warp 0 keeps it).
-struct Team {
+struct ClusterTeam {
+    static constexpr bool kGrid = false;
     int rank, size;
     Shared* sh;
     long long budget;  // clock64 cycles a wait may take
@@ -108,29 +138,21 @@ struct Team {
         sync();
     }
 
-    // Orders every CTA's shared-memory writes before any CTA's following gathers.
+    // Orders every CTA's writes of the gathered vector before any CTA's following gathers.
     __device__ __forceinline__ void sync() const {
         if (size == 1) __syncthreads();
         else cluster_barrier();
     }
+
+    // No CTA leaves while another may still gather from it.
+    __device__ __forceinline__ void finish() const { sync(); }
 
     // Totals over the cluster of Q values per thread: tot[k] = total of value k NRHS + lane,
     // on lanes < NRHS of warp 0 (which then sets the scalar state; a block barrier follows).
     template <int Q, int NRHS>
     __device__ __forceinline__ void reduce(double (&v)[Q], double (&tot)[Q / NRHS]) {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double y[Q];
-#pragma unroll
-            for (int q = 0; q < Q; ++q) y[q] = __shfl_xor_sync(0xffffffffu, v[q], o);
-#pragma unroll
-            for (int q = 0; q < Q; ++q) v[q] += y[q];
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int q = 0; q < Q; ++q) sh->warp[q * kWarps + wid] = v[q];
-        }
+        warp_sums(v, sh);
         __syncthreads();
         if (wid != 0) return;
         // lane q sums value q over the warps, and the partials over the CTAs below
@@ -176,23 +198,105 @@ struct Team {
     }
 };
 
+// The CTAs of one cooperative launch, one per SM. The counter only grows: a barrier is
+// complete when it reaches the number of arrivals so far.
+struct GridTeam {
+    static constexpr bool kGrid = true;
+    int rank, size;
+    Shared* sh;
+    long long budget;
+    unsigned* count;   // arrivals, zeroed before the launch
+    int* err;          // set when a wait expired; every other wait then gives up
+    double* part;      // [2][kMaxQ][size]
+    unsigned target, uses;
+
+    __device__ void init() {
+        if (threadIdx.x == 0) sh->fail = 0;
+        target = uses = 0;
+        __syncthreads();
+    }
+
+    // One thread: arrive (releasing what the block wrote), and wait for every CTA.
+    __device__ __forceinline__ void arrive_and_wait() {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        unsigned seen;
+        const long long t0 = clock64();
+        for (unsigned poll = 1;; ++poll) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+            if ((int)(seen - target) >= 0) return;
+            if (poll % 64 == 0 && (*(volatile int*)err != 0 || clock64() - t0 > budget)) break;
+        }
+        atomicCAS(err, 0, 5 /*KCFD_TIMEOUT*/);
+        sh->fail = 1;
+    }
+
+    __device__ __forceinline__ void sync() {
+        __syncthreads();
+        target += size;
+        if (threadIdx.x == 0) arrive_and_wait();
+        __syncthreads();
+    }
+
+    __device__ __forceinline__ void finish() const {}
+
+    // As ClusterTeam::reduce, the partials through global memory.
+    template <int Q, int NRHS>
+    __device__ __forceinline__ void reduce(double (&v)[Q], double (&tot)[Q / NRHS]) {
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        warp_sums(v, sh);
+        __syncthreads();
+        target += size;
+        // a half of `part` is written again two reductions on, which no CTA starts before
+        // every CTA has read these partials
+        double* slots = part + (size_t)(uses++ & 1u) * kMaxQ * size;
+        if (wid == 0) {
+            if (lane < Q) __stcg(slots + lane * size + rank, tree_sum<kWarps>(sh->warp + lane * kWarps));
+            __syncwarp();
+            if (lane == 0) arrive_and_wait();
+        }
+        __syncthreads();
+        // warp w sums values w, w + kWarps, ... over the CTAs, all its loads in flight together
+#pragma unroll
+        for (int q0 = 0; q0 < Q; q0 += kWarps) {
+            const int q = q0 + wid;
+            if (q < Q) {
+                double s[kMaxGrid / 32];
+#pragma unroll
+                for (int j = 0; j < kMaxGrid / 32; ++j) {
+                    const int at = lane + 32 * j;
+                    s[j] = at < size ? __ldcg(slots + q * size + at) : 0.0;
+                }
+                double total = 0.0;
+#pragma unroll
+                for (int j = 0; j < kMaxGrid / 32; ++j) total += s[j];
+                total = warp_sum(total);
+                if (lane == 0) sh->total[q] = total;
+            }
+        }
+        __syncthreads();
+        const int c = threadIdx.x < NRHS ? threadIdx.x : 0;
+#pragma unroll
+        for (int k = 0; k < Q / NRHS; ++k) tot[k] = sh->total[k * NRHS + c];
+    }
+};
+
 // The system of one CTA, carved from its dynamic shared memory; kRows local rows.
-template <int NRHS, int PREC, int R>
+template <int NRHS, int PREC, int R, bool GRID>
 struct Store {
     static constexpr int kRows = kBlock * R;
-    double* vec;     // [kRows * NRHS] the gathered vector
+    double* vec;     // [kRows * NRHS] the gathered vector (a cluster's; the grid's is global)
     double* val;     // [width][kRows]
     double* lu;      // [width][kRows] (ILU)
-    uint32_t* col;   // [width][kRows]
+    uint32_t* col;   // [width][kRows] address (cluster) or first element (grid) in the gathered vector
     int* loc;        // [nlev + 1] first local row of each level
     int* lev;        // [nlev + 1] first row of each level
 
     static size_t bytes(int width, int nlev) {
-        return (size_t)kRows * (8 * NRHS + width * (PREC == KCFD_PREC_ILU0 ? 20 : 12)) + 8 * (size_t)(nlev + 1);
+        return (size_t)kRows * ((GRID ? 0 : 8 * NRHS) + width * (PREC == KCFD_PREC_ILU0 ? 20 : 12)) + 8 * (size_t)(nlev + 1);
     }
     __device__ Store(char* base, int width, int nlev) {
         vec = (double*)base;
-        val = vec + kRows * NRHS;
+        val = GRID ? vec : vec + kRows * NRHS;
         lu = val + kRows * width;
         col = (uint32_t*)(PREC == KCFD_PREC_ILU0 ? lu + kRows * width : lu);
         loc = (int*)(col + kRows * width);
@@ -212,14 +316,16 @@ __device__ __forceinline__ int level_of(const int* t, int n, int i) {
 }
 
 // A thread's part of the system: rows threadIdx.x + kBlock u, u < R.
-template <int NRHS, int PREC, int R>
+template <int NRHS, int PREC, int R, class Team>
 struct System {
     static constexpr int kRows = kBlock * R;
-    Store<NRHS, PREC, R> s;
+    Store<NRHS, PREC, R, Team::kGrid> s;
     int width, nlev;
+    double* vec;     // the gathered vector; an unused row's part of the grid's lies past the last row
     double di[R];    // 1 / diagonal of A (Jacobi) or of U (ILU), 0 on unused rows
     int lv[R];       // ILU level, -1 on unused rows
     int dk[R];       // position of the diagonal in the row (ILU)
+    int gi[R];       // matrix row (grid only)
 
     // The matrix row of local row t, -1 for an unused one.
     __device__ __forceinline__ int row_of(const Team& tm, int t, int& l) const {
@@ -236,10 +342,20 @@ struct System {
         return i >= 0 && a.perm ? a.perm[i] : i;
     }
 
-    // y[u] = (A g) of the thread's rows, g the gathered vector, entries summed in row order;
-    // the gathers of K entries of all R rows are in flight together.
+    // Component 0 of the thread's row u in the gathered vector.
+    __device__ __forceinline__ double* own(int u) const {
+        return vec + (Team::kGrid ? (size_t)gi[u] * NRHS : (size_t)(threadIdx.x + u * kBlock) * NRHS);
+    }
+    __device__ __forceinline__ double get(uint32_t a, int c) const {
+        // grid: a plain load; L1 serves the rows' common neighbours (the barrier before a
+        // gather acquires, which drops what L1 held before it)
+        return Team::kGrid ? vec[a + c] : ld_cluster(a + 8 * c);
+    }
+
+    // acc[u] = (A g) of the thread's rows, entries summed in row order; the gathers of K
+    // entries of all R rows are in flight together.
     __device__ __forceinline__ void spmv(double (&acc)[R][NRHS]) const {
-        constexpr int K = R * NRHS >= 4 ? 2 : 4;
+        constexpr int V = R * NRHS, K = V <= (Team::kGrid ? 3 : 1) ? 8 : V <= (Team::kGrid ? 4 : 3) ? 4 : 2;
 #pragma unroll
         for (int u = 0; u < R; ++u)
 #pragma unroll
@@ -256,7 +372,7 @@ struct System {
                     for (int u = 0; u < R; ++u) {
                         const uint32_t a = col[j * kRows + u * kBlock];
 #pragma unroll
-                        for (int c = 0; c < NRHS; ++c) y[j][u][c] = ld_cluster(a + 8 * c);
+                        for (int c = 0; c < NRHS; ++c) y[j][u][c] = get(a, c);
                     }
                 }
 #pragma unroll
@@ -272,7 +388,36 @@ struct System {
         }
     }
 
-    // acc -= sum over entries [k0, k1) of the thread's row u of lu[k] g[col k].
+    // g = (LU)^-1 q in the gathered vector; the own rows' part also in z. Level 0 of the
+    // forward and the last level of the backward sweep need no other rows; the caller syncs
+    // before anything gathers g.
+    __device__ __forceinline__ void sweeps(Team& tm, const double (&q)[R][NRHS], double (&z)[R][NRHS]) const {
+        const int last = nlev - 1;
+#pragma unroll 1
+        for (int l = 0; l < 2 * nlev - 1; ++l) {
+            const bool fwd = l < nlev;
+            const int level = fwd ? l : 2 * last - l;
+            if (l > 0) tm.sync();
+            double acc[R][NRHS];
+#pragma unroll
+            for (int u = 0; u < R; ++u)
+#pragma unroll
+                for (int c = 0; c < NRHS; ++c) acc[u][c] = fwd ? q[u][c] : z[u][c];
+            if constexpr (Team::kGrid) sweep_rows(level, fwd, acc);
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                if (lv[u] != level) continue;
+                if constexpr (!Team::kGrid) sweep_row(u, fwd ? 0 : dk[u] + 1, fwd ? dk[u] : width, acc[u]);
+                const double d = fwd && level != last ? 1.0 : di[u];
+#pragma unroll
+                for (int c = 0; c < NRHS; ++c) own(u)[c] = z[u][c] = acc[u][c] * d;
+            }
+        }
+    }
+
+    // acc -= sum over entries [k0, k1) of the thread's row u of lu[k] g[col k] (clusters: the
+    // rows of a level one after another, 2,440 cycles for the sweeps of 7,200 triangles
+    // against 2,700 with all in flight).
     __device__ __forceinline__ void sweep_row(int u, int k0, int k1, double (&acc)[NRHS]) const {
         constexpr int K = NRHS == 1 ? 4 : 2;
         const int at = threadIdx.x + u * kBlock;
@@ -284,7 +429,7 @@ struct System {
                 if (k + j < k1) {
                     const uint32_t a = s.col[(k + j) * kRows + at];
 #pragma unroll
-                    for (int c = 0; c < NRHS; ++c) y[j][c] = ld_cluster(a + 8 * c);
+                    for (int c = 0; c < NRHS; ++c) y[j][c] = get(a, c);
                 }
 #pragma unroll
             for (int j = 0; j < K; ++j)
@@ -296,27 +441,44 @@ struct System {
         }
     }
 
-    // g = (LU)^-1 q in the gathered vector; the own rows' part also in z. Level 0 of the
-    // forward and the last level of the backward sweep need no other rows; the caller syncs
-    // before anything gathers g.
-    __device__ __forceinline__ void sweeps(const Team& tm, const double (&q)[R][NRHS], double (&z)[R][NRHS]) const {
-        const int last = nlev - 1;
+    // The same for all the thread's rows of a level, their gathers in flight together (the
+    // grid, where a gather is an L2 read) and without branches: past its last entry a row
+    // repeats it with value 0, and so does, throughout, a row of another level.
+    __device__ __forceinline__ void sweep_rows(int level, bool fwd, double (&acc)[R][NRHS]) const {
+        int at[R], len[R], most = 0;  // first entry's place, entries
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int k0 = fwd ? 0 : dk[u] + 1;
+            len[u] = lv[u] == level ? (fwd ? dk[u] : width) - k0 : 0;
+            at[u] = (len[u] > 0 ? k0 : 0) * kRows + threadIdx.x + u * kBlock;
+            most = max(most, len[u]);
+        }
+        auto batch = [&](auto count, int k) {
+            constexpr int K = count();
+            double y[K][R][NRHS];
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+#pragma unroll
+                for (int u = 0; u < R; ++u) {
+                    const uint32_t a = s.col[at[u] + max(min(k + j, len[u] - 1), 0) * kRows];
+#pragma unroll
+                    for (int c = 0; c < NRHS; ++c) y[j][u][c] = get(a, c);
+                }
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+#pragma unroll
+                for (int u = 0; u < R; ++u) {
+                    const double v = k + j < len[u] ? s.lu[at[u] + (k + j) * kRows] : 0.0;
+#pragma unroll
+                    for (int c = 0; c < NRHS; ++c) acc[u][c] -= v * y[j][u][c];
+                }
+        };
+        constexpr int kStep = R * NRHS <= 4 ? 3 : 1;
+        if (R * NRHS <= 3 && most > 3 && most <= 6) {  // a hex's neighbours at once
+            batch(std::integral_constant<int, R * NRHS <= 3 ? 6 : 1>(), 0);
+        } else {
 #pragma unroll 1
-        for (int l = 0; l < 2 * nlev - 1; ++l) {
-            const bool fwd = l < nlev;
-            const int level = fwd ? l : 2 * last - l;
-            if (l > 0) tm.sync();
-#pragma unroll
-            for (int u = 0; u < R; ++u) {
-                if (lv[u] != level) continue;
-                double acc[NRHS];
-#pragma unroll
-                for (int c = 0; c < NRHS; ++c) acc[c] = fwd ? q[u][c] : z[u][c];
-                sweep_row(u, fwd ? 0 : dk[u] + 1, fwd ? dk[u] : width, acc);
-                const double d = fwd && level != last ? 1.0 : di[u];
-#pragma unroll
-                for (int c = 0; c < NRHS; ++c) s.vec[(threadIdx.x + u * kBlock) * NRHS + c] = z[u][c] = acc[c] * d;
-            }
+            for (int k = 0; k < most; k += kStep) batch(std::integral_constant<int, kStep>(), k);
         }
     }
 
@@ -344,17 +506,22 @@ struct System {
             double d = 0.0;
 #pragma unroll 4
             for (int k = 0; k < width; ++k) {
-                uint32_t adr = remote(v0 + 8 * NRHS * t, tm.rank);  // padding: the own row, value 0
+                // padding: the own row (the grid's unused rows: the one past the last), value 0
+                uint32_t adr = Team::kGrid ? (uint32_t)(i >= 0 ? i : a.n) * NRHS : remote(v0 + 8 * NRHS * t, tm.rank);
                 double v = 0.0, f = 0.0;
                 if (k < len) {
                     const int j = __ldg(a.indices + kb + k);
                     v = a.vals64[kb + k];
                     if (PREC == KCFD_PREC_ILU0) f = lu[kb + k];
                     if (PREC == KCFD_PREC_JACOBI && j == i) d += v;
-                    const int l = nlev == 1 ? 0 : level_of(s.lev, nlev, j);
-                    const int per = s.loc[l + 1] - s.loc[l];
-                    const int at = j - s.lev[l], rk = at / per;
-                    adr = remote(v0 + 8 * NRHS * (s.loc[l] + at - rk * per), rk);
+                    if (Team::kGrid) {
+                        adr = (uint32_t)j * NRHS;
+                    } else {
+                        const int l = nlev == 1 ? 0 : level_of(s.lev, nlev, j);
+                        const int per = s.loc[l + 1] - s.loc[l];
+                        const int at = j - s.lev[l], rk = at / per;
+                        adr = remote(v0 + 8 * NRHS * (s.loc[l] + at - rk * per), rk);
+                    }
                 }
                 s.val[k * kRows + t] = v;
                 s.col[k * kRows + t] = adr;
@@ -363,6 +530,7 @@ struct System {
             di[u] = 0.0;
             lv[u] = -1;
             dk[u] = 0;
+            gi[u] = i >= 0 ? i : a.n;
             if (i >= 0 && PREC == KCFD_PREC_JACOBI)  // batched systems are set up here
                 di[u] = a.dinv ? ((const double*)a.dinv)[i] : (fabs(d) > 1e-30 ? 1.0 / d : 0.0);
             if (i >= 0 && PREC == KCFD_PREC_ILU0) {
@@ -416,8 +584,8 @@ struct Scalars {
 
 // The iteration, from x and b (in t), with the scalar formulas and tests of bicgstab_body
 // (solver.cu). Returns false when a wait expired.
-template <int NRHS, int PREC, int R>
-__device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R>& S, const SolveArgs& a, int maxiter,
+template <int NRHS, int PREC, int R, class Team>
+__device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R, Team>& S, const SolveArgs& a, int maxiter,
                                         double (&x)[R][NRHS], double (&t)[R][NRHS], Scalars& sc) {
     constexpr bool kPrec = PREC != KCFD_PREC_NONE;
     Shared& sh = *tm.sh;
@@ -431,7 +599,7 @@ __device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R>& S
 #pragma unroll
         for (int u = 0; u < R; ++u)
 #pragma unroll
-            for (int c = 0; c < NRHS; ++c) S.s.vec[(threadIdx.x + u * kBlock) * NRHS + c] = y[u][c];
+            for (int c = 0; c < NRHS; ++c) S.own(u)[c] = y[u][c];
     };
     auto publish = [&](int flags) {  // the lane's scalars, to the block
         sh.al[lane] = sc.alpha;
@@ -624,9 +792,11 @@ __device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R>& S
 }
 
 // FP64 solve on chip, with the true-residual passes of solve_fp64 (solver.cu).
-template <int NRHS, int PREC, int R>
-__device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* store) {
-    System<NRHS, PREC, R> S{Store<NRHS, PREC, R>(store, width, a.nlev), width, a.nlev};
+// gvec: the grid's gathered vector, (n + 1) NRHS elements.
+template <int NRHS, int PREC, int R, class Team>
+__device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* store, double* gvec = nullptr) {
+    System<NRHS, PREC, R, Team> S{Store<NRHS, PREC, R, Team::kGrid>(store, width, a.nlev), width, a.nlev};
+    S.vec = Team::kGrid ? gvec : S.s.vec;
     S.load(tm, a);
     double x[R][NRHS], t[R][NRHS];
 #pragma unroll
@@ -646,7 +816,7 @@ __device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* sto
 #pragma unroll
             for (int c = 0; c < NRHS; ++c) t[u][c] = o >= 0 ? a.b[(size_t)o * NRHS + c] : 0.0;
         }
-        ok = iterate<NRHS, PREC, R>(tm, S, a, a.maxiter - used, x, t, sc);
+        ok = iterate<NRHS, PREC, R, Team>(tm, S, a, a.maxiter - used, x, t, sc);
         if (threadIdx.x == 0) {
             tm.sh->status = sc.status;
             tm.sh->iters = sc.iters;
@@ -670,7 +840,7 @@ __device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* sto
         if (a.status_out) a.status_out[c] = ok ? sc.status : 5 /*KCFD_TIMEOUT*/;
         if (a.relres_out) a.relres_out[c] = sc.bnorm > 0 ? sc.rnorm / sc.bnorm : 0.0;
     }
-    if (a.ctl.err && tm.rank == 0 && threadIdx.x == 0) *a.ctl.err = ok ? 0 : 5 /*KCFD_TIMEOUT*/;
+    if (!Team::kGrid && a.ctl.err && tm.rank == 0 && threadIdx.x == 0) *a.ctl.err = ok ? 0 : 5 /*KCFD_TIMEOUT*/;
 }
 
 }  // namespace res

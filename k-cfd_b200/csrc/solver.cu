@@ -27,8 +27,9 @@
 //    ranges, the lower part of a row is exactly its columns left of the diagonal, and
 //    the forward / backward sweeps read contiguous memory. b and x are permuted on
 //    entry and exit inside the same launch.
-//  * FP64 systems that fit the shared memory of a thread-block cluster (up to 32,768 rows)
-//    are solved there, when the team is chosen automatically (resident.cuh).
+//  * FP64 systems that fit on chip -- a thread-block cluster's shared memory and registers
+//    (up to 32,768 rows) or the whole GPU's (up to about 300,000) -- are solved there, when
+//    the team is chosen automatically (resident.cuh).
 //  * Large FP64 systems run on the graph engine instead (team 3, graph_engine.cuh):
 //    the same iteration as lean phase kernels in one CUDA graph with a device-side
 //    WHILE loop. A solve issued while its stream is being captured falls back to the
@@ -2012,13 +2013,13 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
         }
     }
     // team and launch shape
-    // auto: up to 40,000 unknowns FP64 systems that fit run on chip (resident.cuh, below);
-    // the others, and every mixed solve, on one CTA (tiny systems) or the persistent grid
-    // kernel; the graph engine takes the larger FP64 systems. Measured per Krylov iteration
-    // (Jacobi, one right-hand side, 64^2 cavity p'): one CTA 28 us, the grid kernel 20 us,
-    // the graph engine 25 us, on chip 3.9 us (16 CTAs, one row a thread); with ILU(0) on a
-    // 7,200-triangle channel 40 us on the grid kernel, 6.9 us on chip; 32,400 rows (8 rows
-    // a thread) 7.1 us on chip. A caller that runs many small solves concurrently (the
+    // auto: FP64 systems that fit run on chip (resident.cuh, below), whatever their team; the
+    // others, and every mixed solve, on one CTA (tiny systems) or the persistent grid kernel up
+    // to 40,000 unknowns, and on the graph engine above. Measured per Krylov iteration (one
+    // right-hand side; grid kernel or engine, then on chip): 64^2 cavity p', Jacobi 20 and 3.9
+    // us; 7,200 triangles, ILU(0) 40 and 6.9; 40,000 quads, Jacobi 27 and 10.7, ILU(0) 40 and
+    // 18; 110,592 hexes 30 and 11.5, 45 and 22.5; 216,000 hexes 36 and 13.8, 49 and 34.
+    // A caller that runs many small solves concurrently (the
     // served loop) asks for one CTA explicitly, so that they overlap.
     int team = (amg || cg) ? 3 : opts->team;
     if (team == 0) {
@@ -2192,12 +2193,11 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     } else {
         s->grid = 1;
     }
-    // On chip where it fits: FP64 systems below the graph engine's line, unless the caller
-    // asked for a launch shape (lanes, block, the grid team); one that asked for one CTA
+    // On chip where it fits (FP64), unless the caller asked for a launch shape (lanes, block, the grid team); one that asked for one CTA
     // gets one (256 threads, a lane a row: also by those numbers).
     const bool auto_shape = opts->team == 0 && opts->lanes <= 0 && opts->block <= 0;
     const bool one_cta = opts->team == 1 && opts->lanes <= 1 && (opts->block <= 0 || opts->block == 256);
-    if (!mixed && team <= 2 && (auto_shape || one_cta)) {
+    if (!mixed && !amg && !cg && (auto_shape || one_cta)) {
         const std::vector<int>& rp = s->perm ? pip : ip;
         int width = 0;
         for (int i = 0; i < n; ++i) width = std::max(width, rp[i + 1] - rp[i]);
@@ -2205,7 +2205,9 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     }
     const size_t len = (size_t)n * nrhs;
     bool ok = upload(&s->lev_ptr, lptr);
-    if (s->res.ctas == 0) ok = ok && cudaMalloc(&s->work, 9 * len * vsz) == cudaSuccess;  // on chip: no scratch
+    if (s->res.ctas == 0) ok = ok && cudaMalloc(&s->work, 9 * len * vsz) == cudaSuccess;
+    else if (s->res.scratch > 0) ok = ok && cudaMalloc(&s->work, s->res.scratch * sizeof(double)) == cudaSuccess;
+    if (ok && s->res.scratch > 0) ok = cudaMemset(s->work, 0, s->res.scratch * sizeof(double)) == cudaSuccess;
     if (mixed) ok = ok && cudaMalloc(&s->r64, len * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&s->bar, 2 * sizeof(unsigned)) == cudaSuccess;
     ok = ok && cudaMalloc(&s->err, sizeof(int)) == cudaSuccess;
@@ -2229,7 +2231,7 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
             return e;
         }
     }
-    if (team == 3) {
+    if (team == 3 && s->res.ctas == 0) {
         int e = ge_alloc(s);
         if (!e) e = s->perm ? ge_build_sell(s, pip, pix, psrc, pdiag) : ge_build_sell(s, ip, ix, {}, {});
         if (e) {
@@ -2283,7 +2285,7 @@ int kcfd_solver_setup(kcfd_solver* s, const kcfd_csr_t* A, void* stream) {
         void* k = s->team >= 2 ? (mixed ? (void*)ilu0_factor_grid<float> : (void*)ilu0_factor_grid<double>)
                                : (mixed ? (void*)ilu0_factor_cta<float> : (void*)ilu0_factor_cta<double>);
         if (int e = launch_team(s, k, args, st)) return e;
-        if (s->team == 3) {
+        if (s->team == 3 && s->res.ctas == 0) {
             // the factor's strict lower / upper parts into the engine's SELL copies
             if (mixed) {
                 const float* lu = (const float*)s->lu;
@@ -2314,6 +2316,10 @@ int kcfd_solver_solve(kcfd_solver* s, const kcfd_csr_t* A, const double* b, doub
     a.iters_out = iters;
     a.relres_out = relres;
     a.status_out = status;
+    if (s->res.ctas > 0) {
+        KCFD_CUDA(res::solve(s->res, s->o.nrhs, s->o.precond, a, (double*)s->work, (cudaStream_t)stream));
+        return KCFD_OK;
+    }
     if (s->team == 3) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         KCFD_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
@@ -2321,10 +2327,6 @@ int kcfd_solver_solve(kcfd_solver* s, const kcfd_csr_t* A, const double* b, doub
             return ge_solve(s, A, b, x, iters, relres, status, (cudaStream_t)stream);
         KCFD_REQUIRE(s->o.precond != KCFD_PREC_AMG,
                      "kcfd_solver_solve: an AMG solve runs as its own graph; issue it outside stream capture");
-    }
-    if (s->res.ctas > 0) {
-        KCFD_CUDA(res::solve(s->res, s->o.nrhs, s->o.precond, a, (cudaStream_t)stream));
-        return KCFD_OK;
     }
     void* kern = solve_kernel_ptr(mixed, s->o.nrhs, s->o.precond, s->team >= 2, s->block);
     KCFD_REQUIRE(kern != nullptr, "kcfd_solver_solve: no kernel for this configuration");

@@ -1,5 +1,5 @@
 """On-chip BiCGSTAB (csrc/resident.cuh) against the persistent grid kernel at the sizes where its row split changes:
-one row, one warp, one CTA, ragged last CTAs, the steps to 2, 4 and 8 rows per thread, the largest, and one past it."""
+one row, one warp, one CTA, ragged last CTAs, the steps in rows per thread, the largest of a cluster, the grid form."""
 import numpy as np
 import pytest
 from scipy import sparse
@@ -33,7 +33,7 @@ def greedy_levels(A):
     return lev
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 1025, 4096, 4097, 8193, 11001, 16385, 32768, 32769])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 1025, 4096, 4097, 8193, 11001, 16385, 32768, 32769, 37889, 150001])
 @pytest.mark.parametrize("prec,nrhs", [("none", 1), ("jacobi", 1), ("jacobi", 2), ("jacobi", 3), ("ilu0", 1), ("ilu0", 3)])
 def test_matches_grid_kernel(n, prec, nrhs):
     import torch
