@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_resident(SolveArgs a, int width) 
 // One CTA per SM, for systems beyond a cluster. scratch: the gathered vector, then the
 // partials of the reductions.
 template <int NRHS, int PREC, int R>
-__global__ void __launch_bounds__(kBlock, 1) k_resident_grid(SolveArgs a, int width, double* scratch) {
+__global__ void __launch_bounds__(kBlock, 1) k_resident_grid(SolveArgs a, int width, double* scratch, int comps) {
     extern __shared__ __align__(16) char store[];
     __shared__ Shared sh;
     GridTeam tm;
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_resident_grid(SolveArgs a, int wi
     tm.err = a.ctl.err;
     tm.part = scratch + (size_t)(a.n + 1) * NRHS;
     tm.init();
-    solve_on_chip<NRHS, PREC, R>(tm, a, width, store, scratch);
+    solve_on_chip<NRHS, PREC, R>(tm, a, width, store, scratch, NRHS == 1 ? comps : 1);
 }
 
 // Systems B.order[first + cluster index]: independent solves, one cluster each, scheduled by
@@ -183,20 +183,28 @@ Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max
             return p;
         }
     }
-    // beyond a cluster: one CTA per SM
-    for (int r = 1; r <= 8 && max_ctas > 1; ++r) {
-        const Limits L = limits(nrhs + 4, precond, r);
-        size_t bytes = SIZE_MAX;
-        dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr(), true>::bytes(width, nlev); });
-        if (L.smem == 0 || bytes > (size_t)L.smem || rows_on(L.ctas) > kBlock * r) continue;
-        Plan p;
-        p.ctas = L.ctas;
-        p.grid = true;
-        p.rows_per_thread = r;
-        p.width = width;
-        p.smem = (int)bytes;
-        p.scratch = (size_t)(lev[nlev] + 1) * nrhs + (size_t)2 * kMaxQ * L.ctas;
-        return p;
+    // beyond a cluster: one CTA per SM. Right-hand sides that do not fit together are solved
+    // one after another; with ILU(0) that is slower than the graph engine's joint solve
+    // (216,000 hexes, three right-hand sides, us per iteration: Jacobi 3 x 13.8 against 76,
+    // ILU(0) 3 x 34 against 88).
+    for (int comps : {1, nrhs}) {
+        if (max_ctas == 1 || (comps > 1 && precond == KCFD_PREC_ILU0)) break;
+        const int joint = nrhs / comps;
+        for (int r = 1; r <= 8; ++r) {
+            const Limits L = limits(joint + 4, precond, r);
+            size_t bytes = SIZE_MAX;
+            dispatch(joint, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr(), true>::bytes(width, nlev); });
+            if (L.smem == 0 || bytes > (size_t)L.smem || rows_on(L.ctas) > kBlock * r) continue;
+            Plan p;
+            p.ctas = L.ctas;
+            p.grid = true;
+            p.comps = comps;
+            p.rows_per_thread = r;
+            p.width = width;
+            p.smem = (int)bytes;
+            p.scratch = (size_t)(lev[nlev] + 1) * joint + (size_t)2 * kMaxQ * L.ctas;
+            return p;
+        }
     }
     return Plan();
 }
@@ -234,11 +242,12 @@ cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, doub
     SolveArgs args = a;
     int width = p.width;
     if (p.grid) {
-        void* ptrs[] = {&args, &width, &scratch};
+        int comps = p.comps;
+        void* ptrs[] = {&args, &width, &scratch, &comps};
         cudaError_t e = cudaMemsetAsync(a.ctl.bar, 0, sizeof(unsigned), st);
         if (e == cudaSuccess) e = cudaMemsetAsync(a.ctl.err, 0, sizeof(int), st);
         if (e != cudaSuccess) return e;
-        return cudaLaunchCooperativeKernel(kernel_of(nrhs + 4, precond, p.rows_per_thread), dim3(p.ctas), dim3(kBlock), ptrs,
+        return cudaLaunchCooperativeKernel(kernel_of(nrhs / p.comps + 4, precond, p.rows_per_thread), dim3(p.ctas), dim3(kBlock), ptrs,
                                            p.smem, st);
     }
     void* ptrs[] = {&args, &width};

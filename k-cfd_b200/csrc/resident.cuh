@@ -791,56 +791,63 @@ __device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R, Te
     return true;
 }
 
-// FP64 solve on chip, with the true-residual passes of solve_fp64 (solver.cu).
-// gvec: the grid's gathered vector, (n + 1) NRHS elements.
+// FP64 solve on chip, with the true-residual passes of solve_fp64 (solver.cu). gvec: the
+// grid's gathered vector, (n + 1) NRHS elements. comps > 1 (NRHS 1): that many interleaved
+// right-hand sides, one after another on the same matrix.
 template <int NRHS, int PREC, int R, class Team>
-__device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* store, double* gvec = nullptr) {
+__device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* store, double* gvec = nullptr,
+                              int comps = 1) {
     System<NRHS, PREC, R, Team> S{Store<NRHS, PREC, R, Team::kGrid>(store, width, a.nlev), width, a.nlev};
     S.vec = Team::kGrid ? gvec : S.s.vec;
     S.load(tm, a);
-    double x[R][NRHS], t[R][NRHS];
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-        const int o = S.caller_row(tm, a, threadIdx.x + u * kBlock);
-#pragma unroll
-        for (int c = 0; c < NRHS; ++c) x[u][c] = o >= 0 ? a.x[(size_t)o * NRHS + c] : 0.0;
-    }
-    Scalars sc;
+    const int stride = NRHS * comps;
     const bool verify = NRHS == 1 && a.max_restarts > 0 && a.stop == KCFD_STOP_SCIPY;
-    int used = 0;
-    bool ok = true;
-    for (int pass = 0;; ++pass) {
+    for (int comp = 0; comp < comps; ++comp) {
+        double x[R][NRHS], t[R][NRHS];
 #pragma unroll
         for (int u = 0; u < R; ++u) {
             const int o = S.caller_row(tm, a, threadIdx.x + u * kBlock);
 #pragma unroll
-            for (int c = 0; c < NRHS; ++c) t[u][c] = o >= 0 ? a.b[(size_t)o * NRHS + c] : 0.0;
+            for (int c = 0; c < NRHS; ++c) x[u][c] = o >= 0 ? a.x[(size_t)o * stride + comp + c] : 0.0;
         }
-        ok = iterate<NRHS, PREC, R, Team>(tm, S, a, a.maxiter - used, x, t, sc);
-        if (threadIdx.x == 0) {
-            tm.sh->status = sc.status;
-            tm.sh->iters = sc.iters;
+        Scalars sc;
+        int used = 0;
+        bool ok = true;
+        for (int pass = 0;; ++pass) {
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const int o = S.caller_row(tm, a, threadIdx.x + u * kBlock);
+#pragma unroll
+                for (int c = 0; c < NRHS; ++c) t[u][c] = o >= 0 ? a.b[(size_t)o * stride + comp + c] : 0.0;
+            }
+            ok = iterate<NRHS, PREC, R, Team>(tm, S, a, a.maxiter - used, x, t, sc);
+            if (threadIdx.x == 0) {
+                tm.sh->status = sc.status;
+                tm.sh->iters = sc.iters;
+            }
+            __syncthreads();
+            used += tm.sh->iters;
+            if (!ok || !verify || pass >= kVerifyPasses || tm.sh->status != KCFD_OK || tm.sh->iters == 0 ||
+                used >= a.maxiter)
+                break;
+            tm.sync();  // every gather of the last pass before the next one writes the vector
         }
-        __syncthreads();
-        used += tm.sh->iters;
-        if (!ok || !verify || pass >= kVerifyPasses || tm.sh->status != KCFD_OK || tm.sh->iters == 0 || used >= a.maxiter)
-            break;
-        tm.sync();  // every gather of the last pass before the next one writes the vector
-    }
 #pragma unroll
-    for (int u = 0; u < R; ++u) {
-        const int o = S.caller_row(tm, a, threadIdx.x + u * kBlock);
+        for (int u = 0; u < R; ++u) {
+            const int o = S.caller_row(tm, a, threadIdx.x + u * kBlock);
 #pragma unroll
-        for (int c = 0; c < NRHS; ++c)
-            if (o >= 0) a.x[(size_t)o * NRHS + c] = x[u][c];
+            for (int c = 0; c < NRHS; ++c)
+                if (o >= 0) a.x[(size_t)o * stride + comp + c] = x[u][c];
+        }
+        if (tm.rank == 0 && threadIdx.x < NRHS) {
+            const int c = comp + threadIdx.x;
+            if (a.iters_out) a.iters_out[c] = verify ? used : sc.iters;
+            if (a.status_out) a.status_out[c] = ok ? sc.status : 5 /*KCFD_TIMEOUT*/;
+            if (a.relres_out) a.relres_out[c] = sc.bnorm > 0 ? sc.rnorm / sc.bnorm : 0.0;
+        }
+        if (!Team::kGrid && a.ctl.err && tm.rank == 0 && threadIdx.x == 0) *a.ctl.err = ok ? 0 : 5 /*KCFD_TIMEOUT*/;
+        if (comp + 1 < comps) tm.sync();
     }
-    if (tm.rank == 0 && threadIdx.x < NRHS) {
-        const int c = threadIdx.x;
-        if (a.iters_out) a.iters_out[c] = verify ? used : sc.iters;
-        if (a.status_out) a.status_out[c] = ok ? sc.status : 5 /*KCFD_TIMEOUT*/;
-        if (a.relres_out) a.relres_out[c] = sc.bnorm > 0 ? sc.rnorm / sc.bnorm : 0.0;
-    }
-    if (!Team::kGrid && a.ctl.err && tm.rank == 0 && threadIdx.x == 0) *a.ctl.err = ok ? 0 : 5 /*KCFD_TIMEOUT*/;
 }
 
 }  // namespace res

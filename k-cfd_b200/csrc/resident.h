@@ -18,6 +18,7 @@ struct Plan {
     int ctas = 0;  // 0: the system does not fit on chip
     int rows_per_thread = 0, width = 0, smem = 0;
     bool grid = false;
+    int comps = 1;  // > 1: the right-hand sides one after another
     size_t scratch = 0;
 };
 

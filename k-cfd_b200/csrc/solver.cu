@@ -1143,6 +1143,7 @@ using namespace kcfd;
 
 struct kcfd_solver {
     kcfd_solver_opts_t o;
+    int asked_mode = KCFD_MODE_FP64;  // o.mode is the one it runs in
     int n = 0, nnz = 0;
     int pnnz = 0;  // entries of the permuted matrix (ILU(k): A's plus the fill)
     int grid = 0, block = 256, team = 1, lanes = 8;
@@ -1964,6 +1965,7 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
                  "graph engine (team 0 or 3)");
     auto* s = new kcfd_solver();
     s->o = *opts;
+    s->asked_mode = opts->mode;
     // AMG: the Krylov iteration is FP64 on the graph engine; MIXED selects an FP32
     // multigrid hierarchy (below), so the handle itself runs in FP64
     const int amg_mode = opts->mode;
@@ -1984,8 +1986,8 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     }
     s->sm_count = prop.multiProcessorCount;
     const int nrhs = opts->nrhs;
-    const bool mixed = s->o.mode == KCFD_MODE_MIXED;
-    const size_t vsz = mixed ? sizeof(float) : sizeof(double);
+    bool mixed = s->o.mode == KCFD_MODE_MIXED;
+    size_t vsz = mixed ? sizeof(float) : sizeof(double);
     const int n = A->n, nnz = A->nnz;
     std::vector<int> ip(n + 1), ix(nnz);
     if (cudaMemcpy(ip.data(), A->indptr, ip.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
@@ -2059,6 +2061,24 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     // levels
     std::vector<int> lptr;
     std::vector<int> pip, pix, psrc, pdiag;  // ILU: the level-permuted CSR (host copy)
+    // On chip where it fits, unless the caller asked for a launch shape (lanes, block, a
+    // team); one that asked for one CTA gets one (256 threads, a lane a row: also by those
+    // numbers). A MIXED handle that fits runs in FP64 there: nothing is streamed that FP32
+    // would halve (64^3 cavity, three momentum components: 20 iterations on the MIXED engine
+    // 1,580 us, on chip in FP64 1,100).
+    const bool auto_shape = opts->team == 0 && opts->lanes <= 0 && opts->block <= 0;
+    const bool one_cta = opts->team == 1 && opts->lanes <= 1 && (opts->block <= 0 || opts->block == 256);
+    auto plan_on_chip = [&](const std::vector<int>& rp) {
+        if (amg || cg || !(auto_shape || (one_cta && !mixed))) return;
+        int width = 0;
+        for (int i = 0; i < n; ++i) width = std::max(width, rp[i + 1] - rp[i]);
+        s->res = res::plan(width, nrhs, opts->precond, lptr, one_cta ? 1 : res::kMaxCtas);
+        if (s->res.ctas == 0 || !mixed) return;
+        s->o.mode = KCFD_MODE_FP64;
+        mixed = false;
+        vsz = sizeof(double);
+        s->team = team = ((int64_t)n * nrhs <= 40000) ? team : 3;
+    };
     const int K = opts->precond == KCFD_PREC_ILU0 ? std::max(0, opts->fill_level) : 0;
     if (opts->fill_level < 0) return fail("kcfd_solver_create: fill_level < 0");
     if (opts->precond == KCFD_PREC_ILU0) {
@@ -2146,6 +2166,7 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
         }
         s->pnnz = pip[n];
         s->nlev = nlev;
+        plan_on_chip(pip);
         bool ok = upload(&s->perm, perm) && upload(&s->p_indptr, pip) && upload(&s->p_indices, pix) &&
                   upload(&s->p_src, psrc) && upload(&s->p_diag, pdiag);
         const size_t pn = (size_t)s->pnnz;
@@ -2163,6 +2184,7 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     } else {
         lptr = {0, n};
         s->nlev = 1;
+        plan_on_chip(ip);
     }
     if (cg && opts->precond == KCFD_PREC_ILU0 && s->nlev < 2)
         return fail("kcfd_solver_create: CG with ILU(0) needs a matrix with at least two ILU levels");
@@ -2192,16 +2214,6 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
         s->grid = std::max(1, std::min(g, max_useful));
     } else {
         s->grid = 1;
-    }
-    // On chip where it fits (FP64), unless the caller asked for a launch shape (lanes, block, the grid team); one that asked for one CTA
-    // gets one (256 threads, a lane a row: also by those numbers).
-    const bool auto_shape = opts->team == 0 && opts->lanes <= 0 && opts->block <= 0;
-    const bool one_cta = opts->team == 1 && opts->lanes <= 1 && (opts->block <= 0 || opts->block == 256);
-    if (!mixed && !amg && !cg && (auto_shape || one_cta)) {
-        const std::vector<int>& rp = s->perm ? pip : ip;
-        int width = 0;
-        for (int i = 0; i < n; ++i) width = std::max(width, rp[i + 1] - rp[i]);
-        s->res = res::plan(width, nrhs, opts->precond, lptr, one_cta ? 1 : res::kMaxCtas);
     }
     const size_t len = (size_t)n * nrhs;
     bool ok = upload(&s->lev_ptr, lptr);
@@ -2337,7 +2349,7 @@ int kcfd_solver_solve(kcfd_solver* s, const kcfd_csr_t* A, const double* b, doub
 int kcfd_solver_apply_precond(kcfd_solver* s, const kcfd_csr_t* A, const double* r, double* z, void* stream) {
     KCFD_REQUIRE(s && A && r && z, "kcfd_solver_apply_precond: NULL argument");
     KCFD_REQUIRE(s->o.nrhs == 1, "kcfd_solver_apply_precond: one right-hand side only");
-    KCFD_REQUIRE(s->o.mode == KCFD_MODE_FP64, "kcfd_solver_apply_precond: FP64 handles only");
+    KCFD_REQUIRE(s->asked_mode == KCFD_MODE_FP64 || s->o.precond == KCFD_PREC_AMG, "kcfd_solver_apply_precond: FP64 handles only");
     KCFD_REQUIRE(A->n == s->n && A->nnz == s->nnz, "kcfd_solver_apply_precond: matrix size differs from the bound pattern");
     cudaStream_t st = (cudaStream_t)stream;
     switch (s->o.precond) {

@@ -16,8 +16,8 @@ CUDA graph and replayed.
 Linear solves: the reference calls spsolve; here BiCGSTAB runs to a relative
 residual `rtol` (1e-8 by default) from the current field (momentum) or zero (p').
 precision='mixed' keeps FP64 assembly values for the outer residual and an FP32
-copy (written by the same kernels) for the inner iterations. On large meshes the
-momentum solve runs the graph engine's FP32 form (FP32 vectors and values, FP64
+copy (written by the same kernels) for the inner iterations. A momentum system that fits
+on chip is solved there in FP64; on larger meshes it runs the graph engine's FP32 form (FP32 vectors and values, FP64
 iterate, residual replacement against the FP64 matrix); the p' solve keeps an FP64
 Krylov iteration over an FP32 multigrid hierarchy with precond_p='amg'; with ILU(0)
 or Jacobi it runs FP32 inner iterations with FP64 refinement up to 4,096 cells and
@@ -34,7 +34,7 @@ import numpy as np
 from . import _lib
 from .device_mesh import BoundaryConditions, DeviceMesh
 from .mesh import Mesh, from_fvmesh
-from .solver import DeviceCSR, Solver
+from .solver import DeviceCSR, Solver, mixed_handle
 
 
 class _Field:
@@ -112,11 +112,11 @@ class SIMPLESolver:
                              torch.zeros(nnz, dtype=torch.float32, device=device) if mixed else None)
         self.A_p = DeviceCSR(ip, ix, torch.zeros(nnz, **f64),
                              torch.zeros(nnz, dtype=torch.float32, device=device) if mixed else None)
-        # mixed momentum solves on large meshes: the graph engine's FP32 form (residual
-        # replacement against the FP64 matrix; these systems are well conditioned)
-        team_m = team if team else (3 if (mixed and n * D > 40000) else 0)
-        self.s_m = Solver(self.A_m, precond="jacobi", mode=self.mode, nrhs=D, maxiter=maxiter, rtol=rtol,
-                          team=team_m, lanes=lanes, inner_rtol=inner_rtol, inner_maxiter=inner_maxiter)
+        # mixed momentum solves on meshes beyond the chip: the graph engine's FP32 form
+        # (residual replacement against the FP64 matrix; these systems are well conditioned)
+        make = mixed_handle if mixed else Solver
+        self.s_m = make(self.A_m, precond="jacobi", nrhs=D, maxiter=maxiter, rtol=rtol, team=team, lanes=lanes,
+                        inner_rtol=inner_rtol, inner_maxiter=inner_maxiter)
         levels = None
         if precond_p == "ilu0":
             levels = mesh.cell_color if ilu_order == "color" else mesh.level_natural

@@ -197,6 +197,24 @@ class Solver:
         return e.value
 
 
+# rows up to which a MIXED system may fit on chip (one CTA per SM, 8 rows a thread)
+ON_CHIP_ROWS = 303104
+
+
+def mixed_handle(csr, team=0, nrhs=1, **kw):
+    """A MIXED Solver: on chip where the system fits (FP64 there), else the graph engine's
+    FP32 form above 40,000 unknowns, else the persistent kernel's FP32 inner iterations.
+    An explicit team is taken as it is."""
+    kw["mode"] = _lib.MODE_MIXED
+    if team == 0 and csr.n * nrhs > 40000:
+        if csr.n <= ON_CHIP_ROWS:
+            s = Solver(csr, nrhs=nrhs, **kw)
+            if s.info()["team"] == 3:
+                return s
+        team = 3
+    return Solver(csr, team=team, nrhs=nrhs, **kw)
+
+
 class DeviceGraph:
     """The device work of the kcfd calls issued on `stream` inside the with-block,
     captured as a CUDA graph (kcfd_graph_*); launch() replays it. Allocate (handles,

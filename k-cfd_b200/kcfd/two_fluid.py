@@ -30,7 +30,7 @@ import numpy as np
 from . import _lib
 from .device_mesh import BC_TYPES, DeviceMesh
 from .mesh import Mesh, from_fvmesh
-from .solver import DeviceCSR, Solver
+from .solver import DeviceCSR, Solver, mixed_handle
 
 DIRECT_RTOL = 1e-12
 
@@ -172,20 +172,18 @@ class TwoFluidSolver:
         mode = _lib.MODE_MIXED if precision == "mixed" else _lib.MODE_FP64
         self.precision = precision
         mixed = precision == "mixed"
-        # mixed on large meshes: the graph engine's FP32 form for the momentum, volume
-        # fraction and energy systems (well conditioned: every one has a time term)
-        t1 = 3 if (mixed and n > 40000) else 0
-        tg = 3 if (mixed and n * nd > 40000) else 0
-        self._s1 = Solver(self._A, precond="ilu0", nrhs=1, rtol=rtol, atol=0.0, maxiter=maxiter, levels=levels,
-                          mode=mode, team=t1)
-        self._sg = Solver(self._A, precond="ilu0", nrhs=nd, rtol=rtol, atol=0.0, maxiter=maxiter, levels=levels,
-                          mode=mode, team=tg)
+        # mixed: on chip (FP64) where the momentum, volume fraction and energy systems fit,
+        # the graph engine's FP32 form on larger meshes (well conditioned: every one has a
+        # time term)
+        make = mixed_handle if mixed else Solver
+        self._s1 = make(self._A, precond="ilu0", nrhs=1, rtol=rtol, atol=0.0, maxiter=maxiter, levels=levels)
+        self._sg = make(self._A, precond="ilu0", nrhs=nd, rtol=rtol, atol=0.0, maxiter=maxiter, levels=levels)
         if p_precond == "amg":
             self._sp = Solver(self._A, precond="amg", nrhs=1, rtol=rtol, atol=0.0, maxiter=maxiter, mode=mode)
         elif p_precond == "ilu0":
             # the pinned p' (diag[0] += 1e10) is not well conditioned: in the mixed form
             # it keeps the FP64 Krylov iteration on large meshes
-            self._sp = self._s1 if not t1 else Solver(self._A, precond="ilu0", nrhs=1, rtol=rtol, atol=0.0,
+            self._sp = self._s1 if not (mixed and n > 40000) else Solver(self._A, precond="ilu0", nrhs=1, rtol=rtol, atol=0.0,
                                                       maxiter=maxiter, levels=levels)
         else:
             raise ValueError(f"unknown p' preconditioner {p_precond!r}")

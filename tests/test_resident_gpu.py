@@ -120,3 +120,46 @@ def test_batch_on_chip(prec):
         assert np.linalg.norm(xs[k] - ref) <= 1e-9 * np.linalg.norm(ref)
     for k in (3, 9, 12):
         np.testing.assert_array_equal(solve([k])[0], xs[k])
+
+
+@pytest.mark.parametrize("n,nrhs", [(150001, 3)])
+def test_components_one_after_another(n, nrhs):
+    """Right-hand sides that do not fit on chip together, against each alone."""
+    import torch
+    from kcfd.solver import DeviceCSR, Solver
+    A = system(n, seed=5)
+    d = DeviceCSR.from_scipy(A)
+    b = torch.from_numpy(np.random.default_rng(6).standard_normal((n, nrhs))).cuda()
+    s = Solver(d, precond="jacobi", nrhs=nrhs, rtol=1e-12, maxiter=4000)
+    s.setup(d)
+    x = torch.full_like(b, 0.5)
+    s.solve(d, b, x)
+    assert s.status.tolist() == [0] * nrhs
+    one = Solver(d, precond="jacobi", rtol=1e-12, maxiter=4000)
+    one.setup(d)
+    for c in range(nrhs):
+        xc = torch.full((n,), 0.5, dtype=torch.float64, device="cuda")
+        one.solve(d, b[:, c].contiguous(), xc)
+        assert torch.equal(xc, x[:, c]) and int(one.iters[0]) == int(s.iters[c])
+
+
+@pytest.mark.parametrize("n,nrhs,prec", [(300, 1, "jacobi"), (5000, 2, "ilu0"), (60001, 3, "jacobi")])
+def test_mixed_on_chip(n, nrhs, prec):
+    """A MIXED handle that fits on chip meets the FP64 stopping test, and still refuses the FP64-only calls."""
+    import torch
+    from kcfd import _lib
+    from kcfd.solver import DeviceCSR, Solver
+    A = system(n, seed=8)
+    d = DeviceCSR.from_scipy(A, fp32=True)
+    b = np.random.default_rng(9).standard_normal((n, nrhs))
+    s = Solver(d, precond=prec, mode=_lib.MODE_MIXED, nrhs=nrhs, rtol=1e-11, maxiter=4000,
+               levels=greedy_levels(A) if prec == "ilu0" else None)
+    s.setup(d)
+    x = torch.zeros((n, nrhs), dtype=torch.float64, device="cuda")
+    s.solve(d, torch.from_numpy(b).cuda(), x)
+    assert s.status.tolist() == [0] * nrhs
+    r = A @ x.cpu().numpy() - b
+    assert (np.linalg.norm(r, axis=0) <= 2e-11 * np.linalg.norm(b, axis=0)).all()
+    if nrhs == 1:
+        with pytest.raises(_lib.KcfdError):
+            s.apply_precond(d, x[:, 0].contiguous())
