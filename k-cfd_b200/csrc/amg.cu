@@ -147,64 +147,86 @@ __device__ __forceinline__ double sell_row_dot(const int* __restrict__ off, cons
     return acc;
 }
 
-// acc = sum over CSR row [k0, k1) of val[k] x[col[k]], entries loaded in batches of 8.
-template <typename V, typename T>
-__device__ __forceinline__ double csr_row_dot(int k0, int k1, const int* __restrict__ col, const V* __restrict__ val,
-                                              const T* x) {
-    constexpr int B = 8;
-    double acc = 0.0;
-    for (int k = k0; k < k1; k += B) {
-        int jj[B];
-        double vv[B];
+// B entries of a row (k, k + step, ... below end) in registers: columns (-1: none) and values.
+template <int B, typename V>
+struct Batch {
+    int j[B];
+    double v[B];
+    __device__ __forceinline__ void load(const int* __restrict__ col, const V* __restrict__ val, int k, int step, int end) {
 #pragma unroll
         for (int u = 0; u < B; ++u) {
-            const bool in = k + u < k1;
-            jj[u] = in ? __ldg(col + k + u) : -1;
-            vv[u] = in ? (double)__ldg(val + k + u) : 0.0;
+            const bool in = k + u * step < end;
+            j[u] = in ? __ldg(col + k + u * step) : -1;
+            v[u] = in ? (double)__ldg(val + k + u * step) : 0.0;
         }
-        double xv[B];
+    }
+    template <typename T>
+    __device__ __forceinline__ void add(const T* x, double& acc) const {
+        double y[B];
 #pragma unroll
-        for (int u = 0; u < B; ++u) xv[u] = jj[u] >= 0 ? (double)x[jj[u]] : 0.0;
+        for (int u = 0; u < B; ++u) y[u] = j[u] >= 0 ? (double)x[j[u]] : 0.0;
 #pragma unroll
         for (int u = 0; u < B; ++u)
-            if (jj[u] >= 0) acc += vv[u] * xv[u];
+            if (j[u] >= 0) acc += v[u] * y[u];
     }
-    return acc;
-}
+};
 
-// Lane q of the L lanes sharing row i of a sliced-ELL matrix: the partial sum over the
-// row's entries q, q + L, ... (L = 1: the whole row, entries loaded in batches of 8).
-template <int L, typename V, typename T>
-__device__ __forceinline__ double sell_row_part(const int* __restrict__ off, const int* __restrict__ col,
-                                                const V* __restrict__ val, int i, const T* x, int q) {
-    if (L == 1) return sell_row_dot(off, col, val, i, x);
-    const int sl = i >> 5;
-    const int o0 = __ldg(off + sl), o1 = __ldg(off + sl + 1);
-    const int base = o0 + (i & 31), w = (o1 - o0) >> 5;
-    double acc = 0.0;
-    for (int k = q; k < w; k += L) {
-        const int j = __ldg(col + base + 32 * k);
-        if (j >= 0) acc += (double)__ldg(val + base + 32 * k) * (double)x[j];
-    }
-    return acc;
-}
-
-// Rows of a level handled by groups of L lanes (the small coarse levels, whose rows are
-// long and few, take several lanes per row so that more loads are in flight): f(i,
-// partial sum of row i) for each row, called on every lane with i < n after the L
-// partials are combined by a fixed xor-shuffle tree (lane q == 0 writes). The trip
-// count depends on the warp's first group only, so every lane of a warp runs it.
-template <int L, typename F>
-__device__ __forceinline__ void rows_by_lanes(int n, F f) {
+// Row sums of a level by groups of L lanes (the small coarse levels, whose rows are long and
+// few, take several lanes per row so that more loads are in flight): done(i, sum over row i
+// of val x[col]) on the group's first lane, its L partials combined by a fixed xor-shuffle
+// tree. span(i, first, end) gives the row's entries; lane q takes first + q * unit,
+// + unit * L, .... The trip count depends on the warp's first group only, so every lane of a
+// warp runs it (the shuffles need them all). The pattern and the values do not change during
+// a solve: those of a thread's first row are loaded before the wait for the kernel before
+// this one, which leaves the loop flag and the gathers on the chain after it (a p' step of 262,144
+// hexes, MIXED: 5.30 ms per SIMPLE iteration against 5.59; 40,000 tets 9.12 against 9.33).
+template <int L, int B, typename V, typename T, class Span, class Done>
+__device__ __forceinline__ void lane_rows(int n, int unit, const int* __restrict__ col, const V* __restrict__ val,
+                                          const T* x, const int* active, Span span, Done done) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int q = tid & (L - 1);
     const int groups = (gridDim.x * blockDim.x) / L;
     const int g = tid / L, g0 = (tid & ~31) / L;
+    Batch<B, V> e;
+    int k = 0, end = 0;
+    auto first = [&](int i) {
+        k = end = 0;
+        if (i < n) span(i, k, end);
+        k += q * unit;
+        e.load(col, val, k, unit * L, end);
+    };
+    first(g);
+    pdl_enter();
+    if (inactive(active)) return;
     for (int t = 0; g0 + t * groups < n; ++t) {
         const int i = g + t * groups;
-        f(i, q);
+        if (t > 0) first(i);
+        double s = 0.0;
+        for (;;) {
+            e.add(x, s);
+            k += B * unit * L;
+            if (k >= end) break;
+            e.load(col, val, k, unit * L, end);
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (i < n && q == 0) done(i, s);
     }
 }
+
+// Entries of row i of a sliced-ELL matrix (unit 32) and of a CSR (unit 1).
+__device__ __forceinline__ void sell_span(const int* __restrict__ off, int i, int& k, int& end) {
+    k = __ldg(off + (i >> 5)) + (i & 31);
+    end = __ldg(off + (i >> 5) + 1);
+}
+__device__ __forceinline__ void csr_span(const int* __restrict__ ip, int i, int& k, int& end) {
+    k = __ldg(ip + i);
+    end = __ldg(ip + i + 1);
+}
+
+// Entries in flight per lane: a 7-point row at once; fewer where lanes share a row.
+template <int L>
+constexpr int batch_of() { return L == 1 ? 8 : 4; }
 
 // ------------------------------------------------------------------ cycle kernels --
 // Pre-smoothing from a zero guess and the residual: x = sd b, r = b - W b (W = omega A D^-1).
@@ -212,63 +234,23 @@ template <typename V, typename TI, int L = 1>
 __global__ void __launch_bounds__(256) k_pre(int n, const int* __restrict__ off, const int* __restrict__ col,
                                              const V* __restrict__ W, const V* __restrict__ sd, const TI* b, V* x,
                                              V* r, const int* active) {
-    pdl_enter();
-    if (inactive(active)) return;
-    rows_by_lanes<L>(n, [&](int i, int q) {
-        double wb = i < n ? sell_row_part<L>(off, col, W, i, b, q) : 0.0;
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) wb += __shfl_xor_sync(0xffffffffu, wb, o);
-        if (i < n && q == 0) {
+    lane_rows<L, batch_of<L>()>(
+        n, 32, col, W, b, active, [&](int i, int& k, int& end) { sell_span(off, i, k, end); },
+        [&](int i, double wb) {
             const double bi = (double)b[i];
             x[i] = (V)((double)__ldg(sd + i) * bi);
             r[i] = (V)(bi - wb);
-        }
-    });
+        });
 }
 
 // Restriction bc = P^T r (P^T in CSR). A coarse row gathers the fine rows of its
-// smoothed aggregate (about 24 on 3D hexes), so L lanes share a row: lane q takes the
-// entries q, q + L, ... (the lanes of a row read consecutive entries), then a fixed
-// xor-shuffle tree sums the L partials.
+// smoothed aggregate (about 24 on 3D hexes), so L lanes share a row (the lanes of a row read
+// consecutive entries).
 template <typename V, int L>
 __global__ void __launch_bounds__(256) k_restrict(int nc, const int* __restrict__ rip, const int* __restrict__ rix,
                                                   const V* __restrict__ R, const V* r, V* bc, const int* active) {
-    pdl_enter();
-    if (inactive(active)) return;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int q = threadIdx.x & (L - 1);
-    const int groups = (gridDim.x * blockDim.x) / L;
-    const int g = tid / L, g0 = (tid & ~31) / L;  // this lane's row group, the warp's first
-    // the trip count depends on the warp's first group only, so every lane of a warp
-    // runs every trip (the shuffles need them all)
-    for (int t = 0; g0 + t * groups < nc; ++t) {
-        const int I = g + t * groups;
-        const bool row = I < nc;
-        double acc = 0.0;
-        if (row) {
-            // four entries per lane in flight: columns and values first, then the gathers
-            const int k0 = __ldg(rip + I), k1 = __ldg(rip + I + 1);
-            for (int k = k0 + q; k < k1; k += 4 * L) {
-                int jj[4];
-                double vv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool in = k + u * L < k1;
-                    jj[u] = in ? __ldg(rix + k + u * L) : -1;
-                    vv[u] = in ? (double)__ldg(R + k + u * L) : 0.0;
-                }
-                double xv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) xv[u] = jj[u] >= 0 ? (double)r[jj[u]] : 0.0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (jj[u] >= 0) acc += vv[u] * xv[u];
-            }
-        }
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (row && q == 0) bc[I] = (V)acc;
-    }
+    lane_rows<L, 4>(nc, 1, rix, R, r, active, [&](int i, int& k, int& end) { csr_span(rip, i, k, end); },
+                    [&](int i, double s) { bc[i] = (V)s; });
 }
 
 // Coarsest level: y = C b with C the dense inverse, one warp per row.
@@ -291,10 +273,8 @@ __global__ void __launch_bounds__(256) k_coarse(int nc, const V* __restrict__ C,
 template <typename V>
 __global__ void __launch_bounds__(256) k_prolong(int n, const int* __restrict__ pip, const int* __restrict__ pix,
                                                  const V* __restrict__ P, const V* yc, V* x, const int* active) {
-    pdl_enter();
-    if (inactive(active)) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        x[i] = (V)((double)x[i] + csr_row_dot(__ldg(pip + i), __ldg(pip + i + 1), pix, P, yc));
+    lane_rows<1, 8>(n, 1, pix, P, yc, active, [&](int i, int& k, int& end) { csr_span(pip, i, k, end); },
+                    [&](int i, double s) { x[i] = (V)((double)x[i] + s); });
 }
 
 // Post-smoothing: y = x + sd (b - A x).
@@ -302,14 +282,9 @@ template <typename V, typename TI, typename TO, int L = 1>
 __global__ void __launch_bounds__(256) k_post(int n, const int* __restrict__ off, const int* __restrict__ col,
                                               const V* __restrict__ A, const V* __restrict__ sd, const TI* b,
                                               const V* x, TO* y, const int* active) {
-    pdl_enter();
-    if (inactive(active)) return;
-    rows_by_lanes<L>(n, [&](int i, int q) {
-        double ax = i < n ? sell_row_part<L>(off, col, A, i, x, q) : 0.0;
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
-        if (i < n && q == 0) y[i] = (TO)((double)x[i] + (double)__ldg(sd + i) * ((double)b[i] - ax));
-    });
+    lane_rows<L, batch_of<L>()>(
+        n, 32, col, A, x, active, [&](int i, int& k, int& end) { sell_span(off, i, k, end); },
+        [&](int i, double ax) { y[i] = (TO)((double)x[i] + (double)__ldg(sd + i) * ((double)b[i] - ax)); });
 }
 
 // ------------------------------------------------------------------ set-up kernels --
