@@ -129,12 +129,26 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Rows per thread and per step of the vector kernels: U rows spaced by the grid
-// stride, all loads issued before any store (memory-level parallelism).
+// The vector kernels run over the n * NRHS values as one flat range, U values per thread and
+// step spaced by the grid stride, all loads issued before any store (memory-level
+// parallelism). Rounding the stride down to a multiple of NRHS leaves every thread on one
+// right-hand side (flat(): its first value, stride and right-hand side; up to NRHS - 1
+// threads of the grid stay idle), so its coefficients are scalars and a warp's accesses are
+// consecutive. One row of NRHS values per thread instead reads every NRHS-th value per
+// instruction and keeps fewer loads in flight (three components, 2.1M hexes, Jacobi: one SIMPLE
+// iteration 24.5 ms against 25.0; g_s 39 us, g_xr 65). 32 unsigned bits hold every index whose
+// vectors fit the device (ten of 2^32 values do not).
+constexpr int kIlp = 4;    // g_p, g_s
+constexpr int kIlpXr = 2;  // g_xr: 48 registers, 5 resident CTAs per SM (four: 77 registers, 3 CTAs;
+                           // 194.5 against 191.2 us per p' iteration)
+
 template <int NRHS>
-struct Ilp {
-    static constexpr int U = NRHS == 1 ? 4 : (NRHS == 2 ? 2 : 1);
-};
+__device__ __forceinline__ bool flat(unsigned& q0, unsigned& stride, int& c) {
+    q0 = blockIdx.x * blockDim.x + threadIdx.x;
+    stride = gridDim.x * blockDim.x / NRHS * NRHS;
+    c = q0 % NRHS;
+    return q0 < stride;
+}
 
 // Block partial -> partial array; the last block to arrive sums all partials in a
 // fixed order and returns true with the totals in v (all threads of that block).
@@ -434,54 +448,41 @@ __global__ void __launch_bounds__(kBlock) g_p(ArgsT<T> a) {
     const St& S = *a.st;
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st->trips += 1;
     if (!S.active) return;
-    constexpr int U = Ilp<NRHS>::U;
+    constexpr int U = kIlp;
     const bool gpu = a.stop == KCFD_STOP_GPU;
     const int it = S.it;
-    const int n0 = level0_rows<PREC>(a);
-    double om[NRHS], be[NRHS];
-    int dn[NRHS], rs[NRHS];
-#pragma unroll
-    for (int c = 0; c < NRHS; ++c) {
-        om[c] = S.omega[c];
-        be[c] = S.beta[c];
-        dn[c] = S.done[c];
-        rs[c] = is_mixed<T>() ? S.restart[c] : 0;
-    }
-    const int stride = gridDim.x * blockDim.x;
-    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < a.n; i0 += U * stride) {
-        double R[U][NRHS], P[U][NRHS], V[U][NRHS], D[U];
+    unsigned q0, stride;
+    int c;
+    const bool in = flat<NRHS>(q0, stride, c);
+    const double om = S.omega[c], be = S.beta[c];
+    const bool rs = is_mixed<T>() && S.restart[c];
+    if (!in || S.done[c]) return;
+    const unsigned m = (unsigned)a.n * NRHS, m0 = (unsigned)level0_rows<PREC>(a) * NRHS;
+    for (; q0 < m; q0 += U * stride) {
+        double R[U], P[U], V[U], D[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * stride;
-            if (i < a.n) {
-                if (PREC == KCFD_PREC_JACOBI) D[u] = (double)__ldg(a.dinv + i);
-#pragma unroll
-                for (int c = 0; c < NRHS; ++c) {
-                    const size_t q = (size_t)i * NRHS + c;
-                    R[u][c] = (double)a.r[q];
-                    P[u][c] = (double)a.p[q];
-                    // level-0 rows: v = A M^-1 p = p (never stored there)
-                    V[u][c] = (i < n0) ? P[u][c] : (double)a.v[q];
-                }
+            const unsigned q = q0 + u * stride;
+            if (q < m) {
+                if (PREC == KCFD_PREC_JACOBI) D[u] = (double)__ldg(a.dinv + q / NRHS);
+                R[u] = (double)a.r[q];
+                P[u] = (double)a.p[q];
+                // level-0 rows: v = A M^-1 p = p (never stored there)
+                V[u] = (q < m0) ? P[u] : (double)a.v[q];
             }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * stride;
-            if (i >= a.n) continue;
-#pragma unroll
-            for (int c = 0; c < NRHS; ++c) {
-                if (dn[c]) continue;
-                const size_t q = (size_t)i * NRHS + c;
-                double pn;
-                if (gpu) pn = R[u][c] + be[c] * (P[u][c] - om[c] * V[u][c]);
-                else if (it == 0 || rs[c]) pn = R[u][c];
-                else pn = (P[u][c] - om[c] * V[u][c]) * be[c] + R[u][c];
-                a.p[q] = (T)pn;
-                if (rs[c]) a.rh[q] = a.r[q];  // restart: rhat = r
-                if (PREC == KCFD_PREC_JACOBI) a.ph[q] = (T)(D[u] * pn);
-                if (PREC == KCFD_PREC_ILU0 && a.nlev == 1) a.ph[q] = (T)pn;  // more levels: the sweeps read p
-            }
+            const unsigned q = q0 + u * stride;
+            if (q >= m) continue;
+            double pn;
+            if (gpu) pn = R[u] + be * (P[u] - om * V[u]);
+            else if (it == 0 || rs) pn = R[u];
+            else pn = (P[u] - om * V[u]) * be + R[u];
+            a.p[q] = (T)pn;
+            if (rs) a.rh[q] = a.r[q];  // restart: rhat = r
+            if (PREC == KCFD_PREC_JACOBI) a.ph[q] = (T)(D[u] * pn);
+            if (PREC == KCFD_PREC_ILU0 && a.nlev == 1) a.ph[q] = (T)pn;  // more levels: the sweeps read p
         }
     }
 }
@@ -603,50 +604,38 @@ __global__ void __launch_bounds__(kBlock) g_s(ArgsT<T> a) {
     pdl_enter();
     St& S = *a.st;
     if (!S.active) return;
-    constexpr int U = Ilp<NRHS>::U;
-    const int n0 = level0_rows<PREC>(a);
-    double al[NRHS];
-    int dn[NRHS];
+    constexpr int U = kIlp;
+    unsigned q0, stride;
+    int c;
+    const bool in = flat<NRHS>(q0, stride, c) && !S.done[c];
+    const double al = S.alpha[c];
+    const unsigned m = (unsigned)a.n * NRHS, m0 = (unsigned)level0_rows<PREC>(a) * NRHS;
+    double ss = 0.0;
+    for (; in && q0 < m; q0 += U * stride) {
+        double R[U], V[U], D[U];
 #pragma unroll
-    for (int c = 0; c < NRHS; ++c) {
-        al[c] = S.alpha[c];
-        dn[c] = S.done[c];
+        for (int u = 0; u < U; ++u) {
+            const unsigned q = q0 + u * stride;
+            if (q < m) {
+                if (PREC == KCFD_PREC_JACOBI) D[u] = (double)__ldg(a.dinv + q / NRHS);
+                R[u] = (double)a.r[q];
+                V[u] = (q < m0) ? (double)a.p[q] : (double)a.v[q];  // v = p on level 0
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned q = q0 + u * stride;
+            if (q >= m) continue;
+            const double sv = R[u] - al * V[u];
+            a.r[q] = (T)sv;
+            if (PREC == KCFD_PREC_JACOBI) a.sh[q] = (T)(D[u] * sv);
+            if (PREC == KCFD_PREC_ILU0 && a.nlev == 1) a.sh[q] = (T)sv;  // more levels: the sweeps read s
+            ss += sv * sv;
+        }
     }
     double red[NRHS];
 #pragma unroll
-    for (int c = 0; c < NRHS; ++c) red[c] = 0.0;
-    const int stride = gridDim.x * blockDim.x;
-    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < a.n; i0 += U * stride) {
-        double R[U][NRHS], V[U][NRHS], D[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * stride;
-            if (i < a.n) {
-                if (PREC == KCFD_PREC_JACOBI) D[u] = (double)__ldg(a.dinv + i);
-#pragma unroll
-                for (int c = 0; c < NRHS; ++c) {
-                    const size_t q = (size_t)i * NRHS + c;
-                    R[u][c] = (double)a.r[q];
-                    V[u][c] = (i < n0) ? (double)a.p[q] : (double)a.v[q];  // v = p on level 0
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * stride;
-            if (i >= a.n) continue;
-#pragma unroll
-            for (int c = 0; c < NRHS; ++c) {
-                if (dn[c]) continue;
-                const size_t q = (size_t)i * NRHS + c;
-                const double sv = R[u][c] - al[c] * V[u][c];
-                a.r[q] = (T)sv;
-                if (PREC == KCFD_PREC_JACOBI) a.sh[q] = (T)(D[u] * sv);
-                if (PREC == KCFD_PREC_ILU0 && a.nlev == 1) a.sh[q] = (T)sv;  // more levels: the sweeps read s
-                red[c] += sv * sv;
-            }
-        }
-    }
+    for (int k = 0; k < NRHS; ++k) red[k] = k == c ? ss : 0.0;
     if (last_block_sum<NRHS>(a, 2, red) && threadIdx.x == 0) {
         const bool gpu = a.stop == KCFD_STOP_GPU;
         int any_left = 0;
@@ -754,59 +743,47 @@ __global__ void __launch_bounds__(kBlock) g_xr(ArgsT<T> a) {
     // unconditional bound on the loop, whatever the state logic does
     if (!a.eager && blockIdx.x == 0 && threadIdx.x == 0 && S.trips > a.maxiter + 2) cudaGraphSetConditional(a.cond, 0u);
     if (!S.active) return;
-    // two rows per thread for one right-hand side: 48 registers, 5 resident CTAs per SM
-    // (four rows: 77 registers, 3 CTAs; measured 194.5 against 191.2 us per p' iteration)
-    constexpr int U = NRHS == 1 ? 2 : Ilp<NRHS>::U;
+    constexpr int U = kIlpXr;
     const bool gpu = a.stop == KCFD_STOP_GPU;
     const T* ph = (PREC == KCFD_PREC_NONE) ? a.p : a.ph;
     const T* sh = (PREC == KCFD_PREC_NONE) ? a.r : a.sh;
-    double al[NRHS], om[NRHS];
-    int dn[NRHS];
+    unsigned q0, stride;
+    int c;
+    const bool in = flat<NRHS>(q0, stride, c) && !S.done[c];
+    const double al = S.alpha[c], om = S.omega[c];
+    const unsigned m = (unsigned)a.n * NRHS, m0 = (unsigned)level0_rows<PREC>(a) * NRHS;
+    double rho = 0.0, rr = 0.0;
+    for (; in && q0 < m; q0 += U * stride) {
+        double X[U], HP[U], HS[U], R[U], TT[U], RH[U];
 #pragma unroll
-    for (int c = 0; c < NRHS; ++c) {
-        al[c] = S.alpha[c];
-        om[c] = S.omega[c];
-        dn[c] = S.done[c];
+        for (int u = 0; u < U; ++u) {
+            const unsigned q = q0 + u * stride;
+            if (q < m) {
+                X[u] = a.x[q];
+                HP[u] = (double)ph[q];
+                HS[u] = (double)sh[q];
+                R[u] = (double)a.r[q];
+                TT[u] = (q < m0) ? R[u] : (double)a.t[q];  // t = s on level 0
+                RH[u] = (double)a.rh[q];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned q = q0 + u * stride;
+            if (q >= m) continue;
+            if (gpu) a.x[q] = X[u] + (al * HP[u] + om * HS[u]);
+            else a.x[q] = (X[u] + al * HP[u]) + om * HS[u];
+            const double rn = R[u] - om * TT[u];
+            a.r[q] = (T)rn;
+            rho += RH[u] * rn;
+            rr += rn * rn;
+        }
     }
     double red[2 * NRHS];
 #pragma unroll
-    for (int k = 0; k < 2 * NRHS; ++k) red[k] = 0.0;
-    const int stride = gridDim.x * blockDim.x;
-    const int n0 = level0_rows<PREC>(a);
-    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < a.n; i0 += U * stride) {
-        double X[U][NRHS], HP[U][NRHS], HS[U][NRHS], R[U][NRHS], TT[U][NRHS], RH[U][NRHS];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * stride;
-            if (i < a.n) {
-#pragma unroll
-                for (int c = 0; c < NRHS; ++c) {
-                    const size_t q = (size_t)i * NRHS + c;
-                    X[u][c] = a.x[q];
-                    HP[u][c] = (double)ph[q];
-                    HS[u][c] = (double)sh[q];
-                    R[u][c] = (double)a.r[q];
-                    TT[u][c] = (i < n0) ? R[u][c] : (double)a.t[q];  // t = s on level 0
-                    RH[u][c] = (double)a.rh[q];
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * stride;
-            if (i >= a.n) continue;
-#pragma unroll
-            for (int c = 0; c < NRHS; ++c) {
-                if (dn[c]) continue;
-                const size_t q = (size_t)i * NRHS + c;
-                if (gpu) a.x[q] = X[u][c] + (al[c] * HP[u][c] + om[c] * HS[u][c]);
-                else a.x[q] = (X[u][c] + al[c] * HP[u][c]) + om[c] * HS[u][c];
-                const double rn = R[u][c] - om[c] * TT[u][c];
-                a.r[q] = (T)rn;
-                red[c] += RH[u][c] * rn;
-                red[NRHS + c] += rn * rn;
-            }
-        }
+    for (int k = 0; k < NRHS; ++k) {
+        red[k] = k == c ? rho : 0.0;
+        red[NRHS + k] = k == c ? rr : 0.0;
     }
     if (last_block_sum<2 * NRHS>(a, 4, red) && threadIdx.x == 0) {
         for (int c = 0; c < NRHS; ++c) {

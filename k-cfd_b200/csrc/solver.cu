@@ -1440,24 +1440,24 @@ struct GeGrid {
 
 template <int NRHS, int PREC, typename T>
 GeGrid ge_grids(int n, int sms, int gmax) {
-    auto g = [&](const void* f, int rows_per_thread) {
+    auto g = [&](const void* f, int per_thread, int64_t items) {
         int occ = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, ge::kBlock, 0) != cudaSuccess || occ < 1) occ = 1;
-        const int64_t per = (int64_t)ge::kBlock * rows_per_thread;
-        const int64_t need = ((int64_t)n + per - 1) / per;
+        const int64_t per = (int64_t)ge::kBlock * per_thread;
+        const int64_t need = (items + per - 1) / per;
         return (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)occ * sms, need, (int64_t)gmax}));
     };
-    constexpr int U = ge::Ilp<NRHS>::U;
+    const int64_t flat = (int64_t)n * NRHS;  // the vector kernels' items
     GeGrid r;
-    r.init = g((const void*)ge::g_init<NRHS, T>, 1);
-    r.p = g((const void*)ge::g_p<NRHS, PREC, T>, U);
-    r.fwd = g((const void*)ge::g_fwd<NRHS, T>, 1);
-    r.bwd = g((const void*)ge::g_bwd<NRHS, T>, 1);
-    r.sv = g((const void*)ge::g_spmv_v<NRHS, PREC, T>, 1);
-    r.s = g((const void*)ge::g_s<NRHS, PREC, T>, U);
-    r.st = g((const void*)ge::g_spmv_t<NRHS, PREC, T>, 1);
-    r.xr = g((const void*)ge::g_xr<NRHS, PREC, T>, NRHS == 1 ? 2 : U);  // g_xr's rows per thread
-    r.rr = ge::is_mixed<T>() ? g((const void*)ge::g_rr<NRHS, PREC, T>, 1) : 0;
+    r.init = g((const void*)ge::g_init<NRHS, T>, 1, n);
+    r.p = g((const void*)ge::g_p<NRHS, PREC, T>, ge::kIlp, flat);
+    r.fwd = g((const void*)ge::g_fwd<NRHS, T>, 1, n);
+    r.bwd = g((const void*)ge::g_bwd<NRHS, T>, 1, n);
+    r.sv = g((const void*)ge::g_spmv_v<NRHS, PREC, T>, 1, n);
+    r.s = g((const void*)ge::g_s<NRHS, PREC, T>, ge::kIlp, flat);
+    r.st = g((const void*)ge::g_spmv_t<NRHS, PREC, T>, 1, n);
+    r.xr = g((const void*)ge::g_xr<NRHS, PREC, T>, ge::kIlpXr, flat);
+    r.rr = ge::is_mixed<T>() ? g((const void*)ge::g_rr<NRHS, PREC, T>, 1, n) : 0;
     return r;
 }
 
