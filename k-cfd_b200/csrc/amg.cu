@@ -74,6 +74,7 @@ struct Level {
     void* rV = nullptr;
     int* bip = nullptr;
     int64_t bnnz = 0;
+    int64_t bprod = 0, cprod = 0;                          // terms of the two products
     double* b64 = nullptr;
     int64_t* bptr = nullptr;                    // B entry -> its products [bptr, bptr+1) in (bx, bp)
     int *bx = nullptr, *bp = nullptr;           // A-entry, P-entry index of each product
@@ -116,36 +117,6 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 __device__ __forceinline__ bool inactive(const int* active) { return active && *(volatile const int*)active == 0; }
-
-// acc = sum_k val[k] x[col[k]] over row i of a sliced-ELL matrix (row order), with the
-// row's columns and values loaded in batches of 8 before the gathers of x.
-template <typename V, typename T>
-__device__ __forceinline__ double sell_row_dot(const int* __restrict__ off, const int* __restrict__ col,
-                                               const V* __restrict__ val, int i, const T* x) {
-    const int sl = i >> 5;
-    const int o0 = __ldg(off + sl), o1 = __ldg(off + sl + 1);
-    const int base = o0 + (i & 31), w = (o1 - o0) >> 5;
-    constexpr int B = 8;
-    double acc = 0.0;
-    for (int k0 = 0; k0 < w; k0 += B) {
-        int jj[B];
-        double vv[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const bool in = k0 + u < w;
-            const int slot = base + (k0 + u) * 32;
-            jj[u] = in ? __ldg(col + slot) : -1;
-            vv[u] = in ? (double)__ldg(val + slot) : 0.0;
-        }
-        double xv[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) xv[u] = jj[u] >= 0 ? (double)x[jj[u]] : 0.0;
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (jj[u] >= 0) acc += vv[u] * xv[u];
-    }
-    return acc;
-}
 
 // B entries of a row (k, k + step, ... below end) in registers: columns (-1: none) and values.
 template <int B, typename V>
@@ -351,19 +322,23 @@ __global__ void k_pow_init(int n, double* v, double* part, unsigned* cnt, double
     grid_sum_to(s, part, cnt, nrm2);
 }
 
-// w = D^-1 A v / ||v||, ||w||^2 (A from the level's sliced-ELL copy).
-template <typename V>
-__global__ void k_pow_step(int n, const int* __restrict__ off, const int* __restrict__ col, const V* __restrict__ sA,
-                           const double* __restrict__ dinv, const double* vin, const double* nrm2_in, double* vout,
-                           double* part, unsigned* cnt, double* nrm2_out) {
+// w = D^-1 A v / ||v||, ||w||^2 (A from the level's sliced-ELL copy; L lanes per row as in
+// the smoothers, whose levels these are: the 31,868-row level of 262,144 hexes took 20 us a
+// step with one thread per row of 30 entries, its 777-row level 32; now 11 and 8).
+template <typename V, int L>
+__global__ void __launch_bounds__(256) k_pow_step(int n, const int* __restrict__ off, const int* __restrict__ col,
+                                                  const V* __restrict__ sA, const double* __restrict__ dinv,
+                                                  const double* vin, const double* nrm2_in, double* vout, double* part,
+                                                  unsigned* cnt, double* nrm2_out) {
     const double sc = 1.0 / sqrt(*nrm2_in);
     double s = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double acc = sell_row_dot(off, col, sA, i, vin);
-        const double w = dinv[i] * (acc * sc);
-        vout[i] = w;
-        s += w * w;
-    }
+    lane_rows<L, batch_of<L>()>(
+        n, 32, col, sA, vin, nullptr, [&](int i, int& k, int& end) { sell_span(off, i, k, end); },
+        [&](int i, double acc) {
+            const double w = dinv[i] * (acc * sc);
+            vout[i] = w;
+            s += w * w;
+        });
     grid_sum_to(s, part, cnt, nrm2_out);
 }
 
@@ -426,21 +401,34 @@ __global__ void k_gather(int m, const int* __restrict__ src, const double* __res
     }
 }
 
-// One entry of a sparse product per thread: out[s] = sum over its products t of
-// x[xi[t]] y[yi[t]], in list order (B = A P: x = A, y = P; A_c = P^T B: x = R, y = B).
-__global__ void k_product(int64_t m, const int64_t* __restrict__ ptr, const int* __restrict__ xi,
-                          const int* __restrict__ yi, const double* __restrict__ x, const double* __restrict__ y,
-                          double* __restrict__ out) {
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < m; s += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t0 = ptr[s], t1 = ptr[s + 1];
+// One entry of a sparse product per group of L lanes: out[s] = sum over its products t of
+// x[xi[t]] y[yi[t]] (B = A P: x = A, y = P; A_c = P^T B: x = R, y = B), lane q taking
+// t = q, q + L, ..., the partials combined by a fixed xor-shuffle tree. The lists grow as the
+// levels shrink: one thread per entry leaves a coarse level with few threads on long serial
+// sums, and neighbouring threads read far apart in the lists.
+template <int L>
+__global__ void __launch_bounds__(256) k_product(int64_t m, const int64_t* __restrict__ ptr,
+                                                 const int* __restrict__ xi, const int* __restrict__ yi,
+                                                 const double* __restrict__ x, const double* __restrict__ y,
+                                                 double* __restrict__ out) {
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = threadIdx.x & (L - 1);
+    const int64_t groups = (int64_t)gridDim.x * blockDim.x / L;
+    // the trip count depends on the warp's first group only (the shuffles need every lane)
+    for (int64_t s0 = (tid & ~31) / L; s0 < m; s0 += groups) {
+        const int64_t s = s0 + (threadIdx.x & 31) / L;
+        int64_t t = 0, t1 = 0;
+        if (s < m) {
+            t = __ldg(ptr + s) + q;
+            t1 = __ldg(ptr + s + 1);
+        }
         double acc = 0.0;
-        int64_t t = t0;
-        for (; t + 4 <= t1; t += 4) {
+        for (; t + 3 * L < t1; t += 4 * L) {
             int xa[4], ya[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                xa[u] = __ldg(xi + t + u);
-                ya[u] = __ldg(yi + t + u);
+                xa[u] = __ldg(xi + t + u * L);
+                ya[u] = __ldg(yi + t + u * L);
             }
             double xv[4], yv[4];
 #pragma unroll
@@ -451,8 +439,10 @@ __global__ void k_product(int64_t m, const int64_t* __restrict__ ptr, const int*
 #pragma unroll
             for (int u = 0; u < 4; ++u) acc += xv[u] * yv[u];
         }
-        for (; t < t1; ++t) acc += __ldg(x + __ldg(xi + t)) * __ldg(y + __ldg(yi + t));
-        out[s] = acc;
+        for (; t < t1; t += L) acc += __ldg(x + __ldg(xi + t)) * __ldg(y + __ldg(yi + t));
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (s < m && q == 0) out[s] = acc;
     }
 }
 
@@ -897,6 +887,24 @@ void launch(K k, int grid, int block, cudaStream_t st, bool pdl, Act... args) {
     cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// The kernel of its family for `lanes` lanes per row.
+template <typename K>
+K by_lanes(int lanes, K k1, K k2, K k4, K k8, K k16, K k32) {
+    return lanes >= 32 ? k32 : lanes == 16 ? k16 : lanes == 8 ? k8 : lanes == 4 ? k4 : lanes == 2 ? k2 : k1;
+}
+
+// One sparse product of m entries and `products` terms: lanes per entry so that a lane keeps
+// at least four terms (one batch of loads). The two products of each level, one lane and
+// now: 262,144 hexes 30 + 51, 33 + 49, 15 + 80 us and 33 + 44, 27 + 19, 8 + 8; 2.1M hexes
+// 202 + 372, 212 + 155, 18 + 108 and 221 + 288, 175 + 96, 15 + 13.
+void product(const kcfd_amg* h, int64_t m, int64_t products, const int64_t* ptr, const int* xi, const int* yi,
+             const double* x, const double* y, double* out, cudaStream_t st) {
+    int lanes = 1;
+    while (lanes < 32 && products >= 4 * 2 * lanes * m) lanes <<= 1;
+    const auto k = by_lanes(lanes, k_product<1>, k_product<2>, k_product<4>, k_product<8>, k_product<16>, k_product<32>);
+    k<<<grid_for(h, m * lanes), 256, 0, st>>>(m, ptr, xi, yi, x, y, out);
+}
+
 template <typename V>
 int setup_t(kcfd_amg* h, const double* vals, cudaStream_t st) {
     const int L = h->nlev;
@@ -913,13 +921,15 @@ int setup_t(kcfd_amg* h, const double* vals, cudaStream_t st) {
             k_omega_gersh<<<1, 1, 0, st>>>(h->rmax, h->omega);
         } else {
             k_diag<<<g, 256, 0, st>>>(lv.n, lv.ip, a, lv.dslot, lv.dinv, nullptr);
-            const int gr = std::min(kRedGrid, g);
+            const int gr = std::min(kRedGrid, grid_for(h, (int64_t)lv.n * lv.slanes));
             k_pow_init<<<gr, 256, 0, st>>>(lv.n, h->powv[0], h->part, h->cnt, h->nrm2);
-            const int gp = resident_grid((const void*)k_pow_step<V>, gr, 256);
+            const auto pk = by_lanes(lv.slanes, k_pow_step<V, 1>, k_pow_step<V, 2>, k_pow_step<V, 4>, k_pow_step<V, 8>,
+                                     k_pow_step<V, 16>, k_pow_step<V, 32>);
+            const int gp = resident_grid((const void*)pk, gr, 256);
             for (int t = 0; t < h->o.power_iters; ++t) {
                 const int a_ = t & 1, b_ = a_ ^ 1;
-                k_pow_step<V><<<gp, 256, 0, st>>>(lv.n, lv.soff, lv.scol, (const V*)lv.sA, lv.dinv, h->powv[a_],
-                                                  h->nrm2 + a_, h->powv[b_], h->part, h->cnt, h->nrm2 + b_);
+                pk<<<gp, 256, 0, st>>>(lv.n, lv.soff, lv.scol, (const V*)lv.sA, lv.dinv, h->powv[a_], h->nrm2 + a_,
+                                       h->powv[b_], h->part, h->cnt, h->nrm2 + b_);
             }
             k_omega_pow<<<1, 1, 0, st>>>(h->nrm2 + (h->o.power_iters & 1), h->omega + l);
         }
@@ -929,8 +939,8 @@ int setup_t(kcfd_amg* h, const double* vals, cudaStream_t st) {
         k_pvals<V><<<grid_for(h, lv.pnnz), 256, 0, st>>>(lv.pnnz, lv.prow, lv.pdiag, lv.plp, lv.pla, a, lv.dinv, om,
                                                          lv.p64, (V*)lv.pV);
         k_gather<V><<<grid_for(h, lv.pnnz), 256, 0, st>>>(lv.pnnz, lv.rsrc, lv.p64, lv.r64, (V*)lv.rV);
-        k_product<<<grid_for(h, lv.bnnz), 256, 0, st>>>(lv.bnnz, lv.bptr, lv.bx, lv.bp, a, lv.p64, lv.b64);
-        k_product<<<grid_for(h, nx.nnz), 256, 0, st>>>(nx.nnz, lv.cptr, lv.cr, lv.cb, lv.r64, lv.b64, nx.a64);
+        product(h, lv.bnnz, lv.bprod, lv.bptr, lv.bx, lv.bp, a, lv.p64, lv.b64, st);
+        product(h, nx.nnz, lv.cprod, lv.cptr, lv.cr, lv.cb, lv.r64, lv.b64, nx.a64, st);
         KCFD_CUDA(cudaGetLastError());
     }
     Level& c = h->lv[L - 1];
@@ -959,14 +969,14 @@ int vcycle_t(const kcfd_amg* h, const double* in, double* out, const int* active
                    (const V*)lv.sd, in, (V*)lv.x, (V*)lv.r, active);
         } else {
             const int L_ = lv.slanes;
-            auto pk = L_ >= 32 ? k_pre<V, V, 32> : L_ == 16 ? k_pre<V, V, 16> : L_ == 8 ? k_pre<V, V, 8>
-                    : L_ == 4 ? k_pre<V, V, 4> : L_ == 2 ? k_pre<V, V, 2> : k_pre<V, V, 1>;
+            const auto pk = by_lanes(L_, k_pre<V, V, 1>, k_pre<V, V, 2>, k_pre<V, V, 4>, k_pre<V, V, 8>, k_pre<V, V, 16>,
+                                     k_pre<V, V, 32>);
             launch(pk, grid_for(h, (int64_t)lv.n * L_), 256, st, pdl, lv.n, (const int*)lv.soff, (const int*)lv.scol,
                    (const V*)lv.sW, (const V*)lv.sd, (const V*)lv.b, (V*)lv.x, (V*)lv.r, active);
         }
         const int gr = grid_for(h, (int64_t)nx.n * lv.rlanes);
-        auto rk = lv.rlanes >= 32 ? k_restrict<V, 32> : lv.rlanes == 16 ? k_restrict<V, 16> : lv.rlanes == 8 ? k_restrict<V, 8>
-                : lv.rlanes == 4 ? k_restrict<V, 4> : lv.rlanes == 2 ? k_restrict<V, 2> : k_restrict<V, 1>;
+        const auto rk = by_lanes(lv.rlanes, k_restrict<V, 1>, k_restrict<V, 2>, k_restrict<V, 4>, k_restrict<V, 8>,
+                                 k_restrict<V, 16>, k_restrict<V, 32>);
         launch(rk, gr, 256, st, pdl, nx.n, (const int*)lv.rip, (const int*)lv.rix, (const V*)lv.rV, (const V*)lv.r,
                (V*)nx.b, active);
     }
@@ -984,8 +994,8 @@ int vcycle_t(const kcfd_amg* h, const double* in, double* out, const int* active
                    (const V*)lv.sA, (const V*)lv.sd, in, (const V*)lv.x, out, active);
         } else {
             const int L_ = lv.slanes;
-            auto qk = L_ >= 32 ? k_post<V, V, V, 32> : L_ == 16 ? k_post<V, V, V, 16> : L_ == 8 ? k_post<V, V, V, 8>
-                    : L_ == 4 ? k_post<V, V, V, 4> : L_ == 2 ? k_post<V, V, V, 2> : k_post<V, V, V, 1>;
+            const auto qk = by_lanes(L_, k_post<V, V, V, 1>, k_post<V, V, V, 2>, k_post<V, V, V, 4>, k_post<V, V, V, 8>,
+                                     k_post<V, V, V, 16>, k_post<V, V, V, 32>);
             launch(qk, grid_for(h, (int64_t)lv.n * L_), 256, st, pdl, lv.n, (const int*)lv.soff, (const int*)lv.scol,
                    (const V*)lv.sA, (const V*)lv.sd, (const V*)lv.b, (const V*)lv.x, (V*)lv.y, active);
         }
@@ -1121,6 +1131,8 @@ int kcfd_amg_create(const kcfd_csr_t* A, const kcfd_amg_opts_t* opts, kcfd_amg**
         lv.nc = na;
         lv.pnnz = t.P.ip[cur.n];
         lv.bnnz = t.B.ip[cur.n];
+        lv.bprod = (int64_t)t.bx.size();
+        lv.cprod = (int64_t)t.cr.size();
         lv.slots = (int64_t)col.size();
         ok = up(h, &lv.soff, off) && up(h, &lv.scol, col) && up(h, &lv.ssrc, src) &&
              alloc(h, &lv.sA, lv.slots * vs) && alloc(h, &lv.sW, lv.slots * vs) && alloc(h, &lv.sd, (size_t)cur.n * vs) &&
