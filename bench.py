@@ -206,11 +206,13 @@ def outer_step_bytes(n, Fi, Fb, nnz, ndim, its_m, its_p, p_precond="amg", amg=No
 
 
 def solve_launches(solver, iters):
-    """Kernels one solve launches: the persistent kernels launch once; the graph
-    engine launches the value fill, init, final and the two copies plus, per loop
-    trip, the phase kernels (5), 2 (nlev - 1) ILU sweeps for each of phat and shat, or
-    two V-cycles (4 kernels per level above the coarsest and the coarse solve)."""
-    if not solver.graph_engine:
+    """Kernels one solve launches: the persistent kernels and the on-chip solves launch
+    once (a system that may fit on chip counts as one: a lower bound where it does not);
+    the graph engine launches the value fill, init, final and the two copies plus, per
+    loop trip, the phase kernels (5), 2 (nlev - 1) ILU sweeps for each of phat and shat,
+    or two V-cycles (4 kernels per level above the coarsest and the coarse solve)."""
+    from kcfd.solver import ON_CHIP_ROWS
+    if not solver.graph_engine or (solver.precond != "amg" and solver.n <= ON_CHIP_ROWS):
         return 1
     info = solver.info()
     body = 5
@@ -223,13 +225,14 @@ def solve_launches(solver, iters):
 
 
 def setup_launches(solver, power_iters=8):
-    """Kernels of one preconditioner set-up: Jacobi 1; ILU(0) permute + factor (+ 2
-    SELL fills on the graph engine); AMG per level above the coarsest 9 (level 0) or
-    10 + power iterations, and 2 for the coarsest."""
+    """Kernels of one preconditioner set-up: Jacobi 1; ILU(0) at least 2 (one per level, or
+    permute + factor; + 2 SELL fills on the graph engine beyond the chip); AMG per level
+    above the coarsest 9 (level 0) or 10 + power iterations, and 2 for the coarsest."""
+    from kcfd.solver import ON_CHIP_ROWS
     if solver.precond == "jacobi":
         return 1
     if solver.precond == "ilu0":
-        return 2 + (2 if solver.graph_engine else 0)
+        return 2 + (2 if solver.graph_engine and solver.n > ON_CHIP_ROWS else 0)
     if solver.precond == "amg":
         L = solver.info()["levels"]
         return (9 if L > 1 else 0) + max(0, L - 2) * (10 + power_iters) + 2
@@ -238,17 +241,12 @@ def setup_launches(solver, power_iters=8):
 
 def launches_per_step(s, its_m, its_p):
     """Kernels of libkcfd launched by one outer iteration (excluding memsets), with
-    the Krylov counts of that iteration."""
-    nci, ncb = s.dm.desc.n_colors_int, s.dm.desc.n_colors_bnd
-    per_colour_pass = nci + ncb
-    gg = per_colour_pass + 1
-    mom = per_colour_pass + 1
-    pp = per_colour_pass + 1
+    the Krylov counts of that iteration. Gradients and assembly are one launch each."""
     n = 2                       # mass flux x2
-    n += gg if s.gU_t is not None else 0
-    n += mom + 2                # momentum assembly, residual norms (2)
-    n += pp + 2                 # p' assembly, norm + record
-    n += gg + 2 + 1             # GG p', correction (2), residual bookkeeping
+    n += 1 if s.gU_t is not None else 0
+    n += 1 + 2                  # momentum assembly, residual norms (2)
+    n += 1 + 2                  # p' assembly, norm + record
+    n += 1 + 2 + 1              # GG p', correction (2), residual bookkeeping
     n += setup_launches(s.s_m) + setup_launches(s.s_p)
     n += solve_launches(s.s_m, its_m)
     n += solve_launches(s.s_p, its_p)
