@@ -186,9 +186,10 @@ class Solver:
 
     @property
     def graph_engine(self):
-        """True when solves run as the handle's own CUDA graph (team 3). Such a solve
-        is not nested into an enclosing stream capture (there it runs on the
-        persistent grid kernel), so callers keep it outside their captures."""
+        """True for a handle of team 3: its solves run as the handle's own CUDA graph, or
+        on chip where the system fits. The graph is not nested into an enclosing
+        stream capture (there such a solve runs on the persistent grid kernel), so
+        callers keep it outside their captures."""
         return self.info()["team"] == 3
 
     def barrier_error(self, stream=None):
