@@ -119,6 +119,15 @@ using Args = ArgsT<double>;
 template <typename T>
 constexpr bool is_mixed() { return std::is_same<T, float>::value; }
 
+// FP64 Jacobi: the loop multiplies by A D^-1 (g_scale, once per solve after g_init), so that
+// phat = D^-1 p and shat = D^-1 s are never stored: g_p and g_s write one vector less, g_xr
+// reads D^-1 for two vectors, 133 of 1,540 MB an iteration with three right-hand sides on
+// 2.1M hexes (one SIMPLE iteration there 23.95 -> 23.20 ms; the scaling costs about two
+// iterations' gain).
+// (MIXED keeps its scaled vectors: the difference form needs A's own row sums.)
+template <int PREC, typename T>
+constexpr bool scaled_a() { return PREC == KCFD_PREC_JACOBI && !is_mixed<T>(); }
+
 // Programmatic dependent launch: the phase kernels of one iteration are launched so
 // that the next kernel's CTAs may be scheduled while this one drains. Each phase
 // kernel first waits for the full completion (and memory visibility) of the kernel
@@ -383,6 +392,15 @@ __global__ void g_fill(int64_t m, const int* __restrict__ src, const TI* __restr
     }
 }
 
+// A D^-1 in place (scaled_a).
+__global__ void g_scale(int64_t m, const int* __restrict__ col, const double* __restrict__ dinv,
+                        double* __restrict__ val) {
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
+        const int j = col[k];
+        if (j >= 0) val[k] *= __ldg(dinv + j);
+    }
+}
+
 // MIXED: the FP32 difference-form copy of A from its FP64 SELL copy (same slots):
 // off-diagonal values rounded, the diagonal slot takes the FP64 row sum (summed in
 // row order) rounded once; padding 0.
@@ -494,6 +512,7 @@ __global__ void __launch_bounds__(kBlock) g_p(ArgsT<T> a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st->trips += 1;
     if (!S.active) return;
     constexpr int U = kIlp;
+    constexpr bool kStore = PREC == KCFD_PREC_JACOBI && !scaled_a<PREC, T>();
     const bool gpu = a.stop == KCFD_STOP_GPU;
     const int it = S.it;
     unsigned q0, stride;
@@ -509,7 +528,7 @@ __global__ void __launch_bounds__(kBlock) g_p(ArgsT<T> a) {
         for (int u = 0; u < U; ++u) {
             const unsigned q = q0 + u * stride;
             if (q < m) {
-                if (PREC == KCFD_PREC_JACOBI) D[u] = (double)__ldg(a.dinv + q / NRHS);
+                if (kStore) D[u] = (double)__ldg(a.dinv + q / NRHS);
                 R[u] = (double)a.r[q];
                 P[u] = (double)a.p[q];
                 // level-0 rows: v = A M^-1 p = p (never stored there)
@@ -526,7 +545,7 @@ __global__ void __launch_bounds__(kBlock) g_p(ArgsT<T> a) {
             else pn = (P[u] - om * V[u]) * be + R[u];
             a.p[q] = (T)pn;
             if (rs) a.rh[q] = a.r[q];  // restart: rhat = r
-            if (PREC == KCFD_PREC_JACOBI) a.ph[q] = (T)(D[u] * pn);
+            if (kStore) a.ph[q] = (T)(D[u] * pn);
             if (PREC == KCFD_PREC_ILU0 && a.nlev == 1) a.ph[q] = (T)pn;  // more levels: the sweeps read p
         }
     }
@@ -594,7 +613,7 @@ __global__ void __launch_bounds__(kBlock) g_spmv_v(ArgsT<T> a) {
     pdl_enter();
     St& S = *a.st;
     if (!S.active) return;
-    const T* ph = (PREC == KCFD_PREC_NONE) ? a.p : a.ph;
+    const T* ph = (PREC == KCFD_PREC_NONE || scaled_a<PREC, T>()) ? a.p : a.ph;
     double red[NRHS];
 #pragma unroll
     for (int c = 0; c < NRHS; ++c) red[c] = 0.0;
@@ -645,6 +664,7 @@ __global__ void __launch_bounds__(kBlock) g_s(ArgsT<T> a) {
     St& S = *a.st;
     if (!S.active) return;
     constexpr int U = kIlp;
+    constexpr bool kStore = PREC == KCFD_PREC_JACOBI && !scaled_a<PREC, T>();
     unsigned q0, stride;
     int c;
     const bool in = flat<NRHS>(q0, stride, c) && !S.done[c];
@@ -657,7 +677,7 @@ __global__ void __launch_bounds__(kBlock) g_s(ArgsT<T> a) {
         for (int u = 0; u < U; ++u) {
             const unsigned q = q0 + u * stride;
             if (q < m) {
-                if (PREC == KCFD_PREC_JACOBI) D[u] = (double)__ldg(a.dinv + q / NRHS);
+                if (kStore) D[u] = (double)__ldg(a.dinv + q / NRHS);
                 R[u] = (double)a.r[q];
                 V[u] = (q < m0) ? (double)a.p[q] : (double)a.v[q];  // v = p on level 0
             }
@@ -668,7 +688,7 @@ __global__ void __launch_bounds__(kBlock) g_s(ArgsT<T> a) {
             if (q >= m) continue;
             const double sv = R[u] - al * V[u];
             a.r[q] = (T)sv;
-            if (PREC == KCFD_PREC_JACOBI) a.sh[q] = (T)(D[u] * sv);
+            if (kStore) a.sh[q] = (T)(D[u] * sv);
             if (PREC == KCFD_PREC_ILU0 && a.nlev == 1) a.sh[q] = (T)sv;  // more levels: the sweeps read s
             ss += sv * sv;
         }
@@ -720,8 +740,8 @@ __global__ void __launch_bounds__(kBlock) g_spmv_t(ArgsT<T> a) {
     }
     const bool active = S.active;
     if (!active && !any_sc) return;
-    const T* ph = (PREC == KCFD_PREC_NONE) ? a.p : a.ph;
-    const T* sh = (PREC == KCFD_PREC_NONE) ? a.r : a.sh;
+    const T* ph = (PREC == KCFD_PREC_NONE || scaled_a<PREC, T>()) ? a.p : a.ph;
+    const T* sh = (PREC == KCFD_PREC_NONE || scaled_a<PREC, T>()) ? a.r : a.sh;
     double red[2 * NRHS];
 #pragma unroll
     for (int k = 0; k < 2 * NRHS; ++k) red[k] = 0.0;
@@ -730,7 +750,11 @@ __global__ void __launch_bounds__(kBlock) g_spmv_t(ArgsT<T> a) {
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
 #pragma unroll
             for (int c = 0; c < NRHS; ++c)
-                if (sc[c]) a.x[(size_t)i * NRHS + c] += al[c] * (double)ph[(size_t)i * NRHS + c];
+                if (sc[c]) {
+                    double h = (double)ph[(size_t)i * NRHS + c];
+                    if (scaled_a<PREC, T>()) h *= (double)__ldg(a.dinv + i);
+                    a.x[(size_t)i * NRHS + c] += al[c] * h;
+                }
         }
     }
     const int n0 = active ? level0_rows<PREC>(a) : 0;
@@ -785,8 +809,8 @@ __global__ void __launch_bounds__(kBlock) g_xr(ArgsT<T> a) {
     if (!S.active) return;
     constexpr int U = kIlpXr;
     const bool gpu = a.stop == KCFD_STOP_GPU;
-    const T* ph = (PREC == KCFD_PREC_NONE) ? a.p : a.ph;
-    const T* sh = (PREC == KCFD_PREC_NONE) ? a.r : a.sh;
+    const T* ph = (PREC == KCFD_PREC_NONE || scaled_a<PREC, T>()) ? a.p : a.ph;
+    const T* sh = (PREC == KCFD_PREC_NONE || scaled_a<PREC, T>()) ? a.r : a.sh;
     unsigned q0, stride;
     int c;
     const bool in = flat<NRHS>(q0, stride, c) && !S.done[c];
@@ -801,8 +825,14 @@ __global__ void __launch_bounds__(kBlock) g_xr(ArgsT<T> a) {
             if (q < m) {
                 X[u] = a.x[q];
                 HP[u] = (double)ph[q];
-                HS[u] = (double)sh[q];
                 R[u] = (double)a.r[q];
+                if (scaled_a<PREC, T>()) {
+                    const double d = (double)__ldg(a.dinv + q / NRHS);
+                    HP[u] *= d;
+                    HS[u] = R[u] * d;
+                } else {
+                    HS[u] = (double)sh[q];
+                }
                 TT[u] = (q < m0) ? R[u] : (double)a.t[q];  // t = s on level 0
                 RH[u] = (double)a.rh[q];
             }

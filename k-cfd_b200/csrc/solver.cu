@@ -1575,6 +1575,10 @@ int ge_eager(kcfd_solver* s, cudaStream_t st) {
         }
     }
     if (!cg) ge::g_init<NRHS, T><<<G.init, ge::kBlock, 0, st>>>(a);
+    if constexpr (ge::scaled_a<PREC, T>()) {
+        if (!cg)
+            ge::g_scale<<<ge_fill_grid(s, s->g.slotsA), 256, 0, st>>>(s->g.slotsA, s->g.A.col, a.dinv, s->g.A.val);
+    }
     KCFD_CUDA(cudaGetLastError());
     constexpr int kChunk = 8;
     for (int trips = 0; trips <= a.maxiter + 2; trips += kChunk) {
@@ -1706,6 +1710,21 @@ int ge_build(kcfd_solver* s, const kcfd_csr_t* A) {
     kp.blockDim = dim3(ge::kBlock);
     kp.kernelParams = args;
     KCFD_CUDA(cudaGraphAddKernelNode(&n_init, g.graph, &n_fill, 1, &kp));
+    if constexpr (ge::scaled_a<PREC, T>()) {
+        if (!cg) {
+            int64_t s_m = g.slotsA;
+            const int* s_col = g.A.col;
+            const double* s_d = a.dinv;
+            double* s_val = g.A.val;
+            void* sargs[] = {&s_m, &s_col, &s_d, &s_val};
+            cudaKernelNodeParams ks = kf;
+            ks.func = (void*)ge::g_scale;
+            ks.kernelParams = sargs;
+            cudaGraphNode_t n_scale;
+            KCFD_CUDA(cudaGraphAddKernelNode(&n_scale, g.graph, &n_init, 1, &ks));
+            n_init = n_scale;
+        }
+    }
     // zero-initialised storage (the struct's default constructor is deleted)
     alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)] = {};
     cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
