@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kBlock) g_init(ArgsT<T> a) {
     }
 }
 
-// p = r + beta (p - omega v) (scipy / GPU-path forms); phat = M^-1 p for Jacobi, or
+// p = r + beta (p - omega v) (scipy / GPU-path forms); phat = M^-1 p for MIXED Jacobi, or
 // phat = p for a single-level ILU (with more levels the sweeps read p itself on
 // level 0).
 template <int NRHS, int PREC, typename T>
@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(kBlock) g_spmv_v(ArgsT<T> a) {
     }
 }
 
-// s = r - alpha v (in r); shat = M^-1 s for Jacobi, shat = s for a single-level ILU
+// s = r - alpha v (in r); shat = M^-1 s for MIXED Jacobi, shat = s for a single-level ILU
 // (with more levels the sweeps read s itself on level 0); ||s||.
 template <int NRHS, int PREC, typename T>
 __global__ void __launch_bounds__(kBlock) g_s(ArgsT<T> a) {

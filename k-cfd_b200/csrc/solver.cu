@@ -1130,8 +1130,8 @@ __device__ void ilu0_factor_body(Team& tm, const SolveArgs& a) {
 // and column -> the eliminated row's bounds -> its upper entries, four dependent loads; the
 // persistent kernel walks it entry by entry through a row in local memory. Measured (set-up of
 // one ILU(0), FP64): 40,000 tets 64 and 37 us, 2,700 quads 31 and 20 (without the loads ahead 53
-// and 23). Many levels
-// (a natural ordering) keep the persistent kernel: there a barrier costs less than a launch.
+// and 23). Many levels (a natural ordering) keep the persistent kernel: there a barrier costs
+// less than a launch.
 constexpr int kShortRow = 8, kFewLevels = 16;
 
 template <typename V>
