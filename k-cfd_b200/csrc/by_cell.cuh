@@ -2,8 +2,9 @@
 //
 // A cell goes over its own faces (cf_ptr / cf_face, ascending reference face id: the
 // reference's summation order), adds up its row's sums in registers and writes each of them
-// once; an off-diagonal entry belongs to one (cell, face) pair, so nothing is written twice
-// and no face colours, atomics or zeroed accumulators are needed. The colour-by-colour
+// once; a row's off-diagonal entries are written by its own thread only, so no face colours,
+// atomics or zeroed accumulators are needed. Faces that lead to the same cell share one entry:
+// within a step a face goes on from the sum of the one before it. The colour-by-colour
 // scatter that this replaces (one launch per colour, kept for meshes without cell lists)
 // reads and rewrites the owner's and the neighbour's sums once per colour, with 8 bytes used
 // of every 32-byte sector. A face's data is read twice, the second time mostly from L2.
@@ -68,7 +69,12 @@ __global__ void __launch_bounds__(256) k_by_cell(kcfd_dmesh_t m, Op op) {
             if (e + u >= e1) break;
             const double add = op.apply(c[u], d[u], acc);
             if constexpr (Op::kOff) {
-                if (c[u].in) op.v[on[u]] = old[u] + add;
+                // an earlier face of this step to the same cell: its sum, not the load before it
+#pragma unroll
+                for (int w = 0; w < u; ++w)
+                    if (c[w].in && on[w] == on[u]) old[u] = old[w];
+                old[u] += add;
+                if (c[u].in) op.v[on[u]] = old[u];
             }
         }
     }
