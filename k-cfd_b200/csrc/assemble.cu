@@ -10,8 +10,8 @@
 //
 // Layout and scatter: faces live on the device colour by colour (no two faces of a
 // colour share a cell). One launch per colour processes its faces with one thread
-// each: off-diagonal coefficients go straight into their CSR slots (face -> slot
-// map, each slot written by exactly one face), and the owner/neighbour sums (aP,
+// each: off-diagonal coefficients are added into their zeroed CSR slots (face -> slot
+// map; faces between the same two cells share a slot), and the owner/neighbour sums (aP,
 // rhs, gradients) are plain read-modify-writes that cannot collide inside a colour
 // -- no atomics, and a fixed colour order makes the sums deterministic. A final cell
 // kernel applies the cell terms (time, relaxation, diagonal, pin).
@@ -92,6 +92,19 @@ __global__ void k_mass_flux(DM m, const int8_t* __restrict__ ut, const double* _
     }
 }
 
+// Off-diagonal entries to zero (colour by colour, each face then adds its term).
+__global__ void k_zero_off(DM m, double* __restrict__ v64) {
+    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < m.Fi; f += gridDim.x * blockDim.x)
+        v64[m.slot_on[f]] = v64[m.slot_no[f]] = 0.0;
+}
+
+// One face's term into its entry; faces of one colour share no cell, so no entry either.
+__device__ __forceinline__ void add_off(double* v64, float* v32, int slot, double add) {
+    const double sum = v64[slot] + add;
+    v64[slot] = sum;
+    if (v32) v32[slot] = (float)sum;
+}
+
 // ------------------------------------------------------------------ momentum ----
 // Internal faces of one colour. MUSCL and non-orthogonal corrections read the
 // Green-Gauss gradients gU [n][D][D] (component-major).
@@ -111,12 +124,8 @@ __global__ void k_mom_int(DM m, int f0, int f1, double mu_f, int lim, const doub
             co = -(Df + fmax(-F, 0.0));
             cn = -(Df + fmax(F, 0.0));
         }
-        v64[m.slot_on[f]] = co;
-        v64[m.slot_no[f]] = cn;
-        if (v32) {
-            v32[m.slot_on[f]] = (float)co;
-            v32[m.slot_no[f]] = (float)cn;
-        }
+        add_off(v64, v32, m.slot_on[f], co);
+        add_off(v64, v32, m.slot_no[f], cn);
         const double pf = 0.5 * (p[o] + p[nb]);
         double add_o[D], add_n[D];
 #pragma unroll
@@ -239,6 +248,37 @@ __global__ void k_mom_cells(DM m, double alpha, double rho, double dt, const dou
     }
 }
 
+// The slots of the off-diagonal entries that a row's faces have stored so far, modulo 32.
+// repeated() becomes true when two faces lead to the same cell (a row spans consecutive slots; in
+// one of more than 32 also by chance).
+struct RowSlots {
+    unsigned seen = 0, again = 0;
+    __device__ __forceinline__ void add(int slot) {
+        const unsigned bit = 1u << (slot & 31);
+        again |= seen & bit;
+        seen |= bit;
+    }
+    __device__ __forceinline__ bool repeated() const { return again != 0; }
+};
+
+// The off-diagonal entries of cell i's row as the sums of its faces' terms off(f, own): for
+// rows where faces share an entry, in place of the last face's term.
+template <class Off>
+__device__ __forceinline__ void sum_row(const DM& m, int i, double* v64, float* v32, Off off) {
+    const int e0 = m.cf_ptr[i], e1 = m.cf_ptr[i + 1];
+    auto entries = [&](auto at) {
+        for (int e = e0; e < e1; ++e) {
+            const int f = m.cf_face[e];
+            if (f >= m.Fi) continue;
+            const bool own = m.owner[f] == i;
+            at(f, own, own ? m.slot_on[f] : m.slot_no[f]);
+        }
+    };
+    entries([&](int, bool, int s) { v64[s] = 0.0; });
+    entries([&](int f, bool own, int s) { v64[s] += off(f, own); });
+    if (v32) entries([&](int, bool, int s) { v32[s] = (float)v64[s]; });
+}
+
 // The momentum system of one cell per thread: the terms of k_mom_int, k_mom_bnd and
 // k_mom_cells over the cell's own faces (ascending reference face id), its sums in registers,
 // every entry of its row written once. In place of one launch per colour, which read and
@@ -260,6 +300,7 @@ __global__ void __launch_bounds__(kThreads)
     if (i >= m.n) return;
     constexpr bool kGrad = MUSCL || NONORTH;
     double ui[D], ci[D], gi[D][D], bi[D], ap = 0.0;
+    RowSlots slots;
     const double pi = p[i];
 #pragma unroll
     for (int c = 0; c < D; ++c) {
@@ -313,6 +354,7 @@ __global__ void __launch_bounds__(kThreads)
             ap += Df + fmax(out, 0.0);
             off = -(Df + fmax(-out, 0.0));
         }
+        slots.add(slot);
         v64[slot] = off;
         if (v32) v32[slot] = (float)off;
         const double pf = 0.5 * (pi + p[j]);
@@ -388,6 +430,11 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int c = 1; c < D; ++c) sum = sum + phys;
     dP[i] = m.vol[i] / fmax(sum / D, 1e-30);
+    if (slots.repeated())
+        sum_row(m, i, v64, v32, [&](int f, bool own) {
+            if (m.dlen[f] < 1e-30) return 0.0;
+            return -(mu_f * m.area[f] / m.dorth[f] + fmax(own ? -mf[f] : mf[f], 0.0));
+        });
 }
 
 // -------------------------------------------------------- pressure correction ---
@@ -405,12 +452,8 @@ __global__ void k_pp_int(DM m, int f0, int f1, double rho, const double* __restr
             b[o] -= mf[f];
             b[nb] += mf[f];
         }
-        v64[m.slot_on[f]] = val;
-        v64[m.slot_no[f]] = val;
-        if (v32) {
-            v32[m.slot_on[f]] = (float)val;
-            v32[m.slot_no[f]] = (float)val;
-        }
+        add_off(v64, v32, m.slot_on[f], val);
+        add_off(v64, v32, m.slot_no[f], val);
     }
 }
 
@@ -455,6 +498,7 @@ __global__ void __launch_bounds__(kThreads)
     if (i >= m.n) return;
     const double di = dP[i];
     double ap = 0.0, bi = 0.0;
+    RowSlots slots;
     const int e1 = m.cf_ptr[i + 1];
     for (int e = m.cf_ptr[i]; e < e1; ++e) {
         const int f = m.cf_face[e];
@@ -476,6 +520,7 @@ __global__ void __launch_bounds__(kThreads)
             bi += own ? -F : F;
         }
         if (pin && i == 0) val = 0.0;  // the pinned row: identity
+        slots.add(slot);
         v64[slot] = val;
         if (v32) v32[slot] = (float)val;
     }
@@ -484,6 +529,11 @@ __global__ void __launch_bounds__(kThreads)
     v64[m.diag_slot[i]] = diag;
     if (v32) v32[m.diag_slot[i]] = (float)diag;
     b[i] = pin && i == 0 ? 0.0 : bi;
+    if (slots.repeated())
+        sum_row(m, i, v64, v32, [&](int f, bool own) {
+            if ((pin && i == 0) || m.dlen[f] < 1e-30) return 0.0;
+            return -(rho * 0.5 * (di + dP[own ? m.neigh[f] : m.owner[f]]) * m.area[f] / m.dorth[f]);
+        });
 }
 
 // ------------------------------------------------------------- Green-Gauss ------
@@ -851,6 +901,7 @@ int kcfd_momentum_assemble(const kcfd_dmesh_t* m, const kcfd_bc_t* bc, const kcf
     // a descriptor without cell lists: colour by colour
     KCFD_CUDA(cudaMemsetAsync(aP, 0, sizeof(double) * d.n, st));
     KCFD_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * d.n * D, st));
+    k_zero_off<<<blocks_for(d.Fi), kThreads, 0, st>>>(d, vals64);
     for_colors(m, true, [&](int f0, int f1, int nb) {
 #define KC_MOM(DD, MU, NO) k_mom_int<DD, MU, NO><<<nb, kThreads, 0, st>>>(d, f0, f1, mu_f, lim, U, p, mf, gradU, aP, b, vals64, vals32)
         if (D == 2) {
@@ -887,6 +938,7 @@ int kcfd_pressure_assemble(const kcfd_dmesh_t* m, const kcfd_bc_t* bc, double rh
     }
     KCFD_CUDA(cudaMemsetAsync(aP, 0, sizeof(double) * d.n, st));
     KCFD_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * d.n, st));
+    k_zero_off<<<blocks_for(d.Fi), kThreads, 0, st>>>(d, vals64);
     for_colors(m, true, [&](int f0, int f1, int nb) {
         k_pp_int<<<nb, kThreads, 0, st>>>(d, f0, f1, rho, dP, mf, aP, b, vals64, vals32);
     });

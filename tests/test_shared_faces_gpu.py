@@ -41,3 +41,63 @@ def test_operators_by_cell(monkeypatch, ndim, k):
     assert m.n_internal_faces == k and m.nnz == 4
     monkeypatch.setattr(test_by_cell_gpu, "meshes", lambda: [("pair", m)])
     test_by_cell_gpu.test_by_cell_equals_colours("pair")
+
+
+@pytest.mark.parametrize("lists", [True, False])
+@pytest.mark.parametrize("ndim,k", CASES)
+def test_simple_systems(ndim, k, lists):
+    """SIMPLE's momentum and p' matrices, by cell and (without cell lists) by colour, against sums over the faces on
+    the host: at most 7 terms of one sign an entry, each rounded a few times."""
+    import ctypes as C
+    import torch
+    from kcfd import _lib
+    from kcfd.device_mesh import BCDesc, DeviceMesh, device_layout
+    m = zigzag_pair(ndim, k)
+    n, D, F, Fb, Fi = m.n_cells, m.ndim, m.n_faces, m.n_boundary_faces, m.n_internal_faces
+    rng = np.random.default_rng(5)
+    dm, lay = DeviceMesh(m), device_layout(m)
+    if not lists:
+        dm.desc.cf_ptr = dm.desc.cf_face = None
+    mf, dP = rng.standard_normal(F), rng.uniform(0.1, 2.0, n)
+
+    def dev(a):
+        return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    def full(*s, dt=torch.float64):  # what the kernels must overwrite
+        return torch.full(s, 7.0, dtype=dt, device="cuda")
+
+    t = {"ut": dev(np.ones(Fb, np.int8)), "ub": dev(rng.standard_normal((Fb, D))), "pt": dev(np.ones(Fb, np.int8)),
+         "pv": dev(rng.standard_normal(Fb)), "U": dev(rng.standard_normal((n, D))), "p": dev(rng.standard_normal(n)),
+         "mf": dev(mf), "dP": dev(dP)}
+    rho, mu = 1.3, 0.02
+    owner, neigh = lay["owner"][:Fi], lay["neigh"]
+    area, dorth, F_ = lay["area"][:Fi], lay["dorth"], mf[:Fi]
+    L, P, st = _lib.lib(), _lib.ptr, _lib.stream_handle()
+    for pinned, single in ((0, True), (1, False)):
+        bc = BCDesc()
+        bc.u_type, bc.u_val, bc.p_type, bc.p_val = (t[q].data_ptr() for q in ("ut", "ub", "pt", "pv"))
+        bc.has_p_dirichlet = 1 - pinned
+        prm = _lib.MomParams()
+        prm.rho, prm.mu, prm.alpha_u, prm.dt, prm.limiter, prm.nonorth = rho, mu, 0.7, 0.0, -1, 0
+        df = mu * area / dorth
+        mom = (-(df + np.maximum(-F_, 0.0)), -(df + np.maximum(F_, 0.0)))
+        pp = -rho * 0.5 * (dP[owner] + dP[neigh]) * area / dorth
+        for what, on, no in (("momentum", *mom), ("pressure", pp, pp)):
+            v64, v32 = full(m.nnz), full(m.nnz, dt=torch.float32) if single else None
+            if what == "momentum":
+                _lib.check(L.kcfd_momentum_assemble(C.byref(dm.desc), C.byref(bc), C.byref(prm), P(t["U"]), None,
+                                                    P(t["p"]), P(t["mf"]), None, P(full(n)), P(v64), P(v32),
+                                                    P(full(n, D)), P(full(n)), st), what)
+            else:
+                _lib.check(L.kcfd_pressure_assemble(C.byref(dm.desc), C.byref(bc), rho, P(t["dP"]), P(t["mf"]), P(full(n)),
+                                                    P(v64), P(v32), P(full(n)), st), what)
+            want = np.zeros(m.nnz)
+            np.add.at(want, lay["slot_on"], on)
+            np.add.at(want, lay["slot_no"], no)
+            if what == "pressure" and pinned:
+                want[m.indptr[0]:m.indptr[1]] = 0.0
+            off = np.setdiff1d(np.arange(m.nnz), m.diag_slot)
+            got = v64.cpu().numpy()
+            np.testing.assert_allclose(got[off], want[off], rtol=16 * np.finfo(np.float64).eps, atol=0, err_msg=what)
+            if single:
+                np.testing.assert_array_equal(v32.cpu().numpy(), got.astype(np.float32))
