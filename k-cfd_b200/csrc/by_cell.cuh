@@ -3,8 +3,8 @@
 // A cell goes over its own faces (cf_ptr / cf_face, ascending reference face id: the
 // reference's summation order), adds up its row's sums in registers and writes each of them
 // once; a row's off-diagonal entries are written by its own thread only, so no face colours,
-// atomics or zeroed accumulators are needed. Faces that lead to the same cell share one entry:
-// within a step a face goes on from the sum of the one before it. The colour-by-colour
+// atomics or zeroed accumulators are needed. Faces that lead to the same cell share one entry;
+// a step that holds two of them adds them one after another. The colour-by-colour
 // scatter that this replaces (one launch per colour, kept for meshes without cell lists)
 // reads and rewrites the owner's and the neighbour's sums once per colour, with 8 bytes used
 // of every 32-byte sector. A face's data is read twice, the second time mostly from L2.
@@ -64,17 +64,28 @@ __global__ void __launch_bounds__(256) k_by_cell(kcfd_dmesh_t m, Op op) {
             }
             d[u] = op.load(m, i, c[u], acc);
         }
+        if constexpr (Op::kOff) {
+            bool shared = false;  // two faces to the same cell (or the padding of a last step)
+#pragma unroll
+            for (int u = 1; u < B; ++u)
+#pragma unroll
+                for (int w = 0; w < u; ++w) shared |= c[u].in && on[w] == on[u];
+            if (shared) {
+#pragma unroll
+                for (int u = 0; u < B; ++u) {
+                    if (e + u >= e1) break;
+                    const double add = op.apply(c[u], d[u], acc);
+                    if (c[u].in) op.v[on[u]] += add;
+                }
+                continue;
+            }
+        }
 #pragma unroll
         for (int u = 0; u < B; ++u) {
             if (e + u >= e1) break;
             const double add = op.apply(c[u], d[u], acc);
             if constexpr (Op::kOff) {
-                // an earlier face of this step to the same cell: its sum, not the load before it
-#pragma unroll
-                for (int w = 0; w < u; ++w)
-                    if (c[w].in && on[w] == on[u]) old[u] = old[w];
-                old[u] += add;
-                if (c[u].in) op.v[on[u]] = old[u];
+                if (c[u].in) op.v[on[u]] = old[u] + add;
             }
         }
     }
