@@ -74,6 +74,16 @@ int  kcfd_device_info(int32_t* sm_count, int32_t* cc_major, int32_t* cc_minor);
  * barriers do, and the context stays usable. With team_size == ctas *err stays 0.  */
 int  kcfd_selftest_barrier(int32_t ctas, int32_t team_size, int64_t budget_cycles, uint32_t* bar, int32_t* err,
                            void* stream);
+/* The same for the teams of the on-chip solves: a thread-block cluster of `ctas` CTAs (1 to 8)
+ * or, with grid != 0, a cooperative launch of as many (1 to 64) goes through a few rounds of
+ * barrier, gather and reduction, whose waits may take budget_cycles (clock64). CTA `late`
+ * (negative: none) reaches the second reduction late_cycles late. status: ctas + 2 int32
+ * (zeroed by the call); status[0 .. ctas) = KCFD_OK, KCFD_BREAKDOWN (a wrong sum) or
+ * KCFD_TIMEOUT of each CTA, the last one the grid's error flag. With late_cycles above the
+ * budget the team gives up: every CTA reports KCFD_TIMEOUT and returns, and the context stays
+ * usable. scratch: 19 * ctas doubles.                                                   */
+int  kcfd_selftest_on_chip(int32_t grid, int32_t ctas, int64_t budget_cycles, int32_t late, int64_t late_cycles,
+                           double* scratch, int32_t* status, void* stream);
 typedef struct kcfd_graph kcfd_graph;
 int  kcfd_graph_capture_begin(void* stream);
 int  kcfd_graph_capture_end(void* stream, kcfd_graph** out);

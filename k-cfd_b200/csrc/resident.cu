@@ -19,8 +19,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_resident(SolveArgs a, int width) 
     tm.sh = &sh;
     tm.budget = a.ctl.budget;
     tm.init();
-    solve_on_chip<NRHS, PREC, R>(tm, a, width, store);
-    tm.finish();
+    tm.finish(solve_on_chip<NRHS, PREC, R>(tm, a, width, store));
 }
 
 // One CTA per SM, for systems beyond a cluster. scratch: the gathered vector, then the
@@ -55,8 +54,64 @@ __global__ void __launch_bounds__(kBlock, 1) k_resident_batch(BatchArgs B, int f
     tm.init();
     SolveArgs a = batch_args<double>(B, B.order[first + id]);
     a.dinv = nullptr;
-    solve_on_chip<1, PREC, R>(tm, a, width, store);
-    tm.finish();
+    tm.finish(solve_on_chip<1, PREC, R>(tm, a, width, store));
+}
+
+// Rounds of a solve's steps on the teams above: a value into the gathered vector, a barrier, a
+// gather from the next CTA, a reduction. CTA `late` comes `delay` cycles late to the second
+// round's reduction. status[rank]: KCFD_OK when every sum was right, KCFD_BREAKDOWN when one
+// was not, KCFD_TIMEOUT when the team gave up.
+template <class Team>
+__device__ bool selftest_rounds(Team& tm, double* vec, int late, long long delay, int* status) {
+    bool right = true;
+    auto rounds = [&]() {
+        for (int round = 0; round < 4; ++round) {
+            double* mine = vec + (Team::kGrid ? tm.rank : 0);
+            if (threadIdx.x == 0) *mine = tm.rank + round;
+            tm.sync();
+            const int next = (tm.rank + 1) % tm.size;
+            double v[1], tot[1];
+            v[0] = threadIdx.x > 0 ? 0.0 : Team::kGrid ? __ldcg(vec + next) : ld_cluster(remote(smem_addr(vec), next));
+            if (round == 1 && tm.rank == late)
+                for (const long long t0 = clock64(); clock64() - t0 < delay;) __nanosleep(1000);
+            tm.template reduce<1, 1>(v, tot);
+            if (threadIdx.x == 0) right = right && tot[0] == tm.size * (0.5 * (tm.size - 1) + round);
+            __syncthreads();
+            if (tm.sh->fail) return false;
+        }
+        return true;
+    };
+    const bool ok = tm.settle(rounds());
+    if (threadIdx.x == 0) status[tm.rank] = !ok ? 5 /*KCFD_TIMEOUT*/ : right ? KCFD_OK : KCFD_BREAKDOWN;
+    return ok;
+}
+
+__global__ void __launch_bounds__(kBlock, 1) k_selftest_cluster(int* status, int late, long long delay, long long budget) {
+    __shared__ Shared sh;
+    __shared__ double vec;
+    ClusterTeam tm;
+    int id;
+    cluster_ids(tm.rank, tm.size, id);
+    tm.sh = &sh;
+    tm.budget = budget;
+    tm.init();
+    tm.finish(selftest_rounds(tm, &vec, late, delay, status));
+}
+
+// scratch: a value per CTA, then the partials; ctl: the counter and the error flag.
+__global__ void __launch_bounds__(kBlock, 1)
+    k_selftest_grid(int* status, int late, long long delay, long long budget, double* scratch, int* ctl) {
+    __shared__ Shared sh;
+    GridTeam tm;
+    tm.rank = blockIdx.x;
+    tm.size = gridDim.x;
+    tm.sh = &sh;
+    tm.budget = budget;
+    tm.count = (unsigned*)ctl;
+    tm.err = ctl + 1;
+    tm.part = scratch + tm.size;
+    tm.init();
+    tm.finish(selftest_rounds(tm, scratch, late, delay, status));
 }
 
 namespace {
@@ -258,3 +313,29 @@ cudaError_t solve(const Plan& p, int nrhs, int precond, const SolveArgs& a, doub
 
 }  // namespace res
 }  // namespace kcfd
+
+extern "C" int kcfd_selftest_on_chip(int32_t grid, int32_t ctas, int64_t budget_cycles, int32_t late, int64_t late_cycles,
+                                     double* scratch, int32_t* status, void* stream) {
+    using namespace kcfd;
+    KCFD_REQUIRE(scratch && status, "kcfd_selftest_on_chip: NULL argument");
+    KCFD_REQUIRE(ctas >= 1 && ctas <= (grid ? 64 : 8) && late < ctas,
+                 "kcfd_selftest_on_chip: 1 to 8 CTAs (grid: 64), late below that");
+    KCFD_REQUIRE(budget_cycles > 0 && budget_cycles <= 4000000000LL && late_cycles >= 0 && late_cycles <= 100000000LL,
+                 "kcfd_selftest_on_chip: budget or delay out of range");
+    cudaStream_t st = (cudaStream_t)stream;
+    long long budget = budget_cycles, delay = late_cycles;
+    KCFD_CUDA(cudaMemsetAsync(status, 0, (ctas + 2) * sizeof(int32_t), st));
+    if (grid) {
+        int* ctl = status + ctas;
+        void* ptrs[] = {&status, &late, &delay, &budget, &scratch, &ctl};
+        KCFD_CUDA(cudaLaunchCooperativeKernel((void*)res::k_selftest_grid, dim3(ctas), dim3(res::kBlock), ptrs, 0, st));
+        return KCFD_OK;
+    }
+    res::Plan p;
+    p.ctas = ctas;
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = res::config(p, st, at);
+    void* ptrs[] = {&status, &late, &delay, &budget};
+    KCFD_CUDA(cudaLaunchKernelExC(&cfg, (void*)res::k_selftest_cluster, ptrs));
+    return KCFD_OK;
+}

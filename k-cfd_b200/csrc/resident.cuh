@@ -26,7 +26,8 @@
 //  * the scalar state of right-hand side c lives in the registers of lane c of warp 0,
 //    which broadcasts what the vector phases need.
 // The hardware keeps the CTAs of a cluster resident together; the waits on an mbarrier are
-// bounded all the same (status KCFD_TIMEOUT).
+// bounded all the same (status KCFD_TIMEOUT). A CTA that gives one up stays until no other can
+// gather from it any more (ClusterTeam::settle).
 //
 // Larger systems take the same iteration on one cooperative launch with a CTA per SM
 // (GridTeam): matrix and vectors on chip as above, the gathered vector in global memory (it
@@ -96,7 +97,9 @@ struct Shared {
     double total[kMaxQ];                 // totals over the grid
     double al[3], om[3], be[3];          // alpha, omega, beta of each right-hand side
     int flags[3];
-    int fail;                            // a wait expired
+    int fail;                            // this CTA gave up a wait
+    int any_fail;                        // cluster: one of its CTAs did
+    int settled[kMaxCtas];               // cluster: CTAs that gather and send no more
     int status, iters;                   // of right-hand side 0, after a pass
 };
 
@@ -119,6 +122,13 @@ __device__ __forceinline__ void warp_sums(double (&v)[Q], Shared* sh) {
 }
 
 // The CTAs of one cluster; `uses` counts reductions (warp 0 keeps it).
+//
+// A wait that expires leaves its CTA without totals, so without the decisions of the others. It
+// tells every CTA (any_fail), sends no more partials, and settles: it goes on meeting the
+// others at their barriers, and stays for their gathers, until each of them has settled too.
+// They do at the latest in their next reduction, which lacks its partials: that wait sees
+// any_fail and gives up. Nothing of this is on the path of a solve whose waits do not expire
+// but the look at any_fail between two polls.
 struct ClusterTeam {
     static constexpr bool kGrid = false;
     int rank, size;
@@ -129,7 +139,8 @@ struct ClusterTeam {
     __device__ void init() {
         for (int i = threadIdx.x; i < kMaxQ * kMaxCtas; i += kBlock) sh->part[0][i] = sh->part[1][i] = 0.0;
         if (threadIdx.x == 0) {
-            sh->fail = 0;
+            sh->fail = sh->any_fail = 0;
+            for (int r = 0; r < kMaxCtas; ++r) sh->settled[r] = 0;
             for (int h = 0; h < 2; ++h)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh->bar[h])) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -144,8 +155,35 @@ struct ClusterTeam {
         else cluster_barrier();
     }
 
-    // No CTA leaves while another may still gather from it.
-    __device__ __forceinline__ void finish() const { sync(); }
+    __device__ void tell(int* flag) const {  // flag = 1 in every CTA
+        const uint32_t at = smem_addr(flag);
+        for (int r = 0; r < size; ++r)
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote(at, r)), "r"(1) : "memory");
+    }
+
+    // The end of a solve, ok: without an expired wait in this CTA. True, in every thread of every
+    // CTA alike, when none expired. No CTA returns while another may gather from it.
+    __device__ bool settle(bool ok) const {
+        if (size == 1) return ok;
+        if (threadIdx.x == 0) tell(&sh->settled[rank]);
+        if (ok) {
+            sync();  // the same barrier for all CTAs whose waits were met; the others meet it too
+            return *(volatile int*)&sh->any_fail == 0;
+        }
+        for (int b = 0, n = 0; n < size && b < 1 << 20; ++b) {
+            sync();
+            n = 0;
+            for (int r = 0; r < size; ++r) n += *(volatile int*)&sh->settled[r];
+        }
+        return false;
+    }
+
+    // Before the CTA ends. When every wait was met no partial is on its way to it. Otherwise some
+    // may be, and nothing counts them any more: one takes below 1,000 cycles, this 1,000 times that.
+    __device__ void finish(bool ok) const {
+        if (ok) return;
+        for (const long long t0 = clock64(); clock64() - t0 < 1000000;) __nanosleep(1000);
+    }
 
     // Totals over the cluster of Q values per thread: tot[k] = total of value k NRHS + lane,
     // on lanes < NRHS of warp 0 (which then sets the scalar state; a block barrier follows).
@@ -179,7 +217,7 @@ struct ClusterTeam {
             }
             uint32_t ok = 0;
             const long long t0 = clock64();
-            for (;;) {
+            for (unsigned poll = 1;; ++poll) {
                 asm volatile(
                     "{ .reg .pred p;\n"
                     "  mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
@@ -187,9 +225,13 @@ struct ClusterTeam {
                     : "=r"(ok)
                     : "r"(bar), "r"(phase)
                     : "memory");
-                if (ok || clock64() - t0 > budget) break;
+                if (ok) break;
+                if (poll % 16 == 0 && (*(volatile int*)&sh->any_fail != 0 || clock64() - t0 > budget)) break;
             }
-            if (!ok) sh->fail = 1;
+            if (!ok) {
+                tell(&sh->any_fail);
+                sh->fail = 1;
+            }
             __syncwarp();
             s = tree_sum<kMaxCtas>(sh->part[h] + q * kMaxCtas);
         }
@@ -237,7 +279,15 @@ struct GridTeam {
         __syncthreads();
     }
 
-    __device__ __forceinline__ void finish() const {}
+    // As ClusterTeam::settle. No CTA reads another's shared memory, so one that gave up leaves by
+    // itself; err then ends the others' waits.
+    __device__ __forceinline__ bool settle(bool ok) {
+        if (!ok) return false;
+        sync();
+        return !sh->fail;
+    }
+
+    __device__ __forceinline__ void finish(bool) const {}
 
     // As ClusterTeam::reduce, the partials through global memory.
     template <int Q, int NRHS>
@@ -583,7 +633,7 @@ struct Scalars {
 };
 
 // The iteration, from x and b (in t), with the scalar formulas and tests of bicgstab_body
-// (solver.cu). Returns false when a wait expired.
+// (solver.cu). Returns false when this CTA gave up a wait.
 template <int NRHS, int PREC, int R, class Team>
 __device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R, Team>& S, const SolveArgs& a, int maxiter,
                                         double (&x)[R][NRHS], double (&t)[R][NRHS], Scalars& sc) {
@@ -793,16 +843,17 @@ __device__ __forceinline__ bool iterate(Team& tm, const System<NRHS, PREC, R, Te
 
 // FP64 solve on chip, with the true-residual passes of solve_fp64 (solver.cu). gvec: the
 // grid's gathered vector, (n + 1) NRHS elements. comps > 1 (NRHS 1): that many interleaved
-// right-hand sides, one after another on the same matrix.
+// right-hand sides, one after another on the same matrix. False when a wait expired.
 template <int NRHS, int PREC, int R, class Team>
-__device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* store, double* gvec = nullptr,
+__device__ bool solve_on_chip(Team& tm, const SolveArgs& a, int width, char* store, double* gvec = nullptr,
                               int comps = 1) {
     System<NRHS, PREC, R, Team> S{Store<NRHS, PREC, R, Team::kGrid>(store, width, a.nlev), width, a.nlev};
     S.vec = Team::kGrid ? gvec : S.s.vec;
     S.load(tm, a);
     const int stride = NRHS * comps;
     const bool verify = NRHS == 1 && a.max_restarts > 0 && a.stop == KCFD_STOP_SCIPY;
-    for (int comp = 0; comp < comps; ++comp) {
+    bool ok = true;
+    for (int comp = 0; comp < comps && ok; ++comp) {
         double x[R][NRHS], t[R][NRHS];
 #pragma unroll
         for (int u = 0; u < R; ++u) {
@@ -812,7 +863,6 @@ __device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* sto
         }
         Scalars sc;
         int used = 0;
-        bool ok = true;
         for (int pass = 0;; ++pass) {
 #pragma unroll
             for (int u = 0; u < R; ++u) {
@@ -832,6 +882,7 @@ __device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* sto
                 break;
             tm.sync();  // every gather of the last pass before the next one writes the vector
         }
+        ok = tm.settle(ok);
 #pragma unroll
         for (int u = 0; u < R; ++u) {
             const int o = S.caller_row(tm, a, threadIdx.x + u * kBlock);
@@ -846,8 +897,8 @@ __device__ void solve_on_chip(Team& tm, const SolveArgs& a, int width, char* sto
             if (a.relres_out) a.relres_out[c] = sc.bnorm > 0 ? sc.rnorm / sc.bnorm : 0.0;
         }
         if (!Team::kGrid && a.ctl.err && tm.rank == 0 && threadIdx.x == 0) *a.ctl.err = ok ? 0 : 5 /*KCFD_TIMEOUT*/;
-        if (comp + 1 < comps) tm.sync();
     }
+    return ok;
 }
 
 }  // namespace res
