@@ -260,6 +260,9 @@ typedef struct {
  * row levels of a multicolour ILU(0) for a matrix that comes without a mesh. Two coupled
  * rows never share a colour.                                                         */
 int kcfd_row_colouring(int32_t n, const int32_t* indptr_host, const int32_t* indices_host, int32_t* colour);
+/* The levels that an ILU(0) handle gives its rows without level_of_row_host: natural order,
+ * one more than the highest level among the rows left of the diagonal (host only).       */
+int kcfd_natural_levels(int32_t n, const int32_t* indptr_host, const int32_t* indices_host, int32_t* level);
 /* ILU(0) ordering: level_of_row_host gives each row's level (e.g. the mesh's cell
  * colouring, or natural-order dependency levels); NULL -> natural-order levels.
  * Coupled rows must lie on different levels. With ILU(0) the handle solves the

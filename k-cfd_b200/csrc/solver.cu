@@ -1319,6 +1319,15 @@ int free_solver(kcfd_solver* s) {
     return KCFD_OK;
 }
 
+// Level of each row in index order: one more than the highest among the rows left of its diagonal.
+void natural_levels(int n, const int* ip, const int* ix, int* lev) {
+    for (int i = 0; i < n; ++i) {
+        lev[i] = 0;
+        for (int k = ip[i]; k < ip[i + 1]; ++k)
+            if (ix[k] < i) lev[i] = std::max(lev[i], lev[ix[k]] + 1);
+    }
+}
+
 // Greedy distance-d colouring of A's symmetrised graph, rows in index order: each row
 // takes the smallest colour not used by any row within d edges of it. With d = k + 1
 // no ILU(k) fill entry joins two rows of one colour (a level-l fill entry (i, j)
@@ -2018,13 +2027,26 @@ void kcfd_graph_destroy(kcfd_graph* g) {
     delete g;
 }
 
-int kcfd_row_colouring(int32_t n, const int32_t* indptr, const int32_t* indices, int32_t* colour) {
-    KCFD_REQUIRE(indptr && indices && colour && n > 0 && indptr[0] == 0, "kcfd_row_colouring: bad pattern");
+static int check_pattern(const char* who, int32_t n, const int32_t* indptr, const int32_t* indices) {
+    KCFD_REQUIRE(indptr && indices && n > 0 && indptr[0] == 0, "%s: bad pattern", who);
     for (int i = 0; i < n; ++i) {
-        KCFD_REQUIRE(indptr[i + 1] >= indptr[i], "kcfd_row_colouring: indptr not monotone at row %d", i);
+        KCFD_REQUIRE(indptr[i + 1] >= indptr[i], "%s: indptr not monotone at row %d", who, i);
         for (int k = indptr[i]; k < indptr[i + 1]; ++k)
-            KCFD_REQUIRE(indices[k] >= 0 && indices[k] < n, "kcfd_row_colouring: column index out of range at %d", k);
+            KCFD_REQUIRE(indices[k] >= 0 && indices[k] < n, "%s: column index out of range at %d", who, k);
     }
+    return KCFD_OK;
+}
+
+int kcfd_natural_levels(int32_t n, const int32_t* indptr, const int32_t* indices, int32_t* level) {
+    KCFD_REQUIRE(level, "kcfd_natural_levels: NULL argument");
+    if (int e = check_pattern("kcfd_natural_levels", n, indptr, indices)) return e;
+    natural_levels(n, indptr, indices, level);
+    return KCFD_OK;
+}
+
+int kcfd_row_colouring(int32_t n, const int32_t* indptr, const int32_t* indices, int32_t* colour) {
+    KCFD_REQUIRE(colour, "kcfd_row_colouring: NULL argument");
+    if (int e = check_pattern("kcfd_row_colouring", n, indptr, indices)) return e;
     const std::vector<int> c = distance_colouring(n, std::vector<int>(indptr, indptr + n + 1),
                                                   std::vector<int>(indices, indices + indptr[n]), 1);
     std::copy(c.begin(), c.end(), colour);
@@ -2179,9 +2201,7 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
         } else if (level_of_row_host) {
             for (int i = 0; i < n; ++i) lev[i] = level_of_row_host[i];
         } else {
-            for (int i = 0; i < n; ++i)
-                for (int k = ip[i]; k < ip[i + 1]; ++k)
-                    if (ix[k] < i) lev[i] = std::max(lev[i], lev[ix[k]] + 1);
+            natural_levels(n, ip.data(), ix.data(), lev.data());
         }
         int nlev = 0;
         for (int i = 0; i < n; ++i) {

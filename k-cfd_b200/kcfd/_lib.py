@@ -81,6 +81,7 @@ SIGNATURES = {
     "kcfd_spmv_f64": (i32, [C.POINTER(Csr), vp, vp, i32, vp]),
     "kcfd_spmv_f32": (i32, [C.POINTER(Csr), vp, vp, i32, vp]),
     "kcfd_row_colouring": (i32, [i32, vp, vp, vp]),
+    "kcfd_natural_levels": (i32, [i32, vp, vp, vp]),
     "kcfd_solver_create": (i32, [C.POINTER(Csr), C.POINTER(SolverOpts), vp, C.POINTER(vp)]),
     "kcfd_solver_destroy": (None, [vp]),
     "kcfd_solver_setup": (i32, [vp, C.POINTER(Csr), vp]),

@@ -21,7 +21,8 @@ device failure raises instead of falling back to the CPU. Semantics kept:
     residual of 1e-12 stands in for spsolve (documented difference). A matrix without
     ILU levels of its own is coloured first: natural-order levels are some hundred
     short dependent steps per sweep (5,000 triangles, whole call: 84 ms against 7.4 ms coloured);
-    they are the second try where the coloured factor does not converge.
+    they are the second try, from x0 again, where the coloured factor does not reach that
+    residual in a bounded number of iterations, and the only one for chain-like matrices.
 system may be the reference's FVMSystem (anything with .to_sparse() and .rhs), a
 kcfd FVMSystem, or a device-assembled kcfd DeviceSystem.
 """
@@ -35,6 +36,9 @@ from . import _lib
 from .solver import DeviceCSR, Solver
 
 DIRECT_RTOL = 1e-12
+# the coloured factor takes more iterations than the natural order's, so its recursive residual
+# drifts further from the true one: it is solved a decade further, and the true one is checked
+COLOURED_RTOL = 1e-13
 SCIPY_DEFAULT_RTOL = 1e-5
 
 
@@ -92,13 +96,46 @@ def _as_device(system):
     return DeviceCSR.from_scipy(A), b, None
 
 
-def _colour_levels(d):
+def _colour_levels(d, ip=None, ix=None):
     """Greedy row colouring of the matrix graph, as ILU(0) levels (kcfd_row_colouring)."""
-    ip, ix = d.indptr.cpu().numpy(), d.indices.cpu().numpy()
+    if ip is None:
+        ip, ix = d.indptr.cpu().numpy(), d.indices.cpu().numpy()
     lev = np.empty(d.n, dtype=np.int32)
     _lib.check(_lib.lib().kcfd_row_colouring(d.n, ip.ctypes.data, ix.ctypes.data, lev.ctypes.data),
                "kcfd_row_colouring")
     return lev
+
+
+def _direct_tries(d, its):
+    """(ILU(0) levels, rtol, iteration limit) in the order that method='direct' tries them.
+
+    A sweep over `depth` natural-order levels costs about as much as depth / 2 coloured
+    iterations of the same system, so the coloured try may take 20 depth of them: those of some
+    ten to forty natural-order iterations (48,400 quads: 439 levels, 3.3 ms a natural iteration
+    against 18 us; 289 coloured iterations against 201). Where the levels hold fewer than four
+    rows on average the graph is close to a chain, whose natural-order factor is close to exact:
+    one iteration, where the coloured one takes hundreds (2,000 rows in a row: 6.1 against 7.2 ms,
+    and a residual of 5e-15 against 3e-12)."""
+    ip, ix = d.indptr.cpu().numpy(), d.indices.cpu().numpy()
+    lev = np.empty(d.n, dtype=np.int32)
+    _lib.check(_lib.lib().kcfd_natural_levels(d.n, ip.ctypes.data, ix.ctypes.data, lev.ctypes.data),
+               "kcfd_natural_levels")
+    depth = int(lev.max()) + 1
+    natural = (None, DIRECT_RTOL, its)
+    if 4 * depth > d.n:
+        return [natural]
+    return [(_colour_levels(d, ip, ix), COLOURED_RTOL, min(its, 200 + 20 * depth)), natural]
+
+
+def _residual_met(d, b, x):
+    """||b - A x|| <= DIRECT_RTOL ||b||, or within the rounding of the residual itself (rows of some
+    eight entries: 8 u (|A| |x| + |b|)), below which no solution can be told from another."""
+    norm = float(b.norm())
+    res = float((b - d.spmv(x)).norm())
+    if res <= DIRECT_RTOL * norm:
+        return True
+    floor = DeviceCSR(d.indptr, d.indices, d.vals64.abs()).spmv(x.abs()) + b.abs()
+    return res <= 4 * np.finfo(np.float64).eps * float(floor.norm())
 
 
 def solve_linear_system(system, x0=None, method="direct", tol=1e-8, maxiter=1000, backend="auto",
@@ -128,24 +165,30 @@ def solve_linear_system(system, x0=None, method="direct", tol=1e-8, maxiter=1000
     if prec == "amg":
         amg_kw = {"amg_max_levels": int(precond_kwargs.pop("max_levels", 0)),
                   "amg_coarse_max": min(int(precond_kwargs.pop("max_coarse", 0)), 256)}
-    tries = [levels] if method != "direct" or levels is not None else [_colour_levels(d), None]
+    first = (levels, rtol_eff, its)
+    tries = [first] if method != "direct" or levels is not None else _direct_tries(d, its)
     x_start = x.clone() if len(tries) > 1 else x
-    for lev in tries:
-        s = Solver(d, precond=prec, stop=_lib.STOP_SCIPY, maxiter=its, rtol=rtol_eff, atol=atol, levels=lev,
+    for k, (lev, rt, limit) in enumerate(tries):
+        s = Solver(d, precond=prec, stop=_lib.STOP_SCIPY, maxiter=limit, rtol=rt, atol=atol, levels=lev,
                    fill_level=fill, **amg_kw)
         s.setup(d)
-        it, rr, st = s.solve(d, b, x)
-        status = int(st[0])
-        if status == _lib.OK or lev is tries[-1]:
+        # a pass from the solution before restarts the recursive residual from the true one
+        for _ in range(1 if k + 1 == len(tries) else 2):
+            it, rr, st = s.solve(d, b, x)
+            status = int(st[0])
+            if status not in (_lib.OK, _lib.MAXITER, _lib.BREAKDOWN):
+                raise _lib.KcfdError(status, "device solve failed")
+            met = status == _lib.OK and (k + 1 == len(tries) or _residual_met(d, b, x))
+            if met or status != _lib.OK:
+                break
+        err = s.barrier_error()
+        if err:
+            raise _lib.KcfdError(err, "device barrier wait expired")
+        if met or k + 1 == len(tries):
             break
         x.copy_(x_start)
     if status == _lib.MAXITER and method == "bicgstab":
         print(f"[bicgstab] 수렴 실패: {int(it[0])} 반복 후 중단")
-    elif status not in (_lib.OK, _lib.MAXITER, _lib.BREAKDOWN):
-        raise _lib.KcfdError(status, "device solve failed")
-    err = s.barrier_error()
-    if err:
-        raise _lib.KcfdError(err, "device barrier wait expired")
     return x.cpu().numpy()
 
 
