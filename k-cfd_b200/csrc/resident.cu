@@ -167,11 +167,20 @@ cudaLaunchConfig_t config(const Plan& p, cudaStream_t st, cudaLaunchAttribute* a
 }
 
 // What the device grants a kernel: dynamic shared memory, and the largest cluster that can be
-// resident at that much. Asked once per device and kernel (the questions take up to a
-// millisecond each).
+// resident at that much. Asked once per device and kernel, and only for one whose rows would
+// hold the system: the questions load the kernel and take up to a millisecond each.
 struct Limits {
     int smem = 0, ctas = 0;
 };
+
+// CTAs of a cooperative launch: one per SM.
+int grid_ctas() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    return std::max(1, std::min(sms, kMaxGrid));
+}
 
 Limits limits(int nrhs, int precond, int r) {
     constexpr int kDevices = 64;
@@ -195,8 +204,7 @@ Limits limits(int nrhs, int precond, int r) {
     Plan p;
     p.smem = optin - (int)fa.sharedSizeBytes;
     if (nrhs > 4) {
-        if (cudaDeviceGetAttribute(&L.ctas, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return Limits();
-        L.ctas = std::min(L.ctas, kMaxGrid);
+        L.ctas = grid_ctas();
         L.smem = p.smem;
         return L;
     }
@@ -224,32 +232,34 @@ Plan plan(int width, int nrhs, int precond, const std::vector<int>& lev, int max
     };
     // the fewest rows per thread first: a thread's rows are done one after another
     for (int r = 1; r <= 8; ++r) {
+        int c = 1;
+        while (c <= max_ctas && rows_on(c) > kBlock * r) ++c;
+        if (c > max_ctas) continue;
         const Limits L = limits(nrhs, precond, r);
         size_t bytes = SIZE_MAX;
         dispatch(nrhs, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr(), false>::bytes(width, nlev); });
-        if (L.smem == 0 || bytes > (size_t)L.smem) continue;
-        for (int c = 1; c <= std::min(max_ctas, L.ctas); ++c) {
-            if (rows_on(c) > kBlock * r) continue;
-            Plan p;
-            p.ctas = c;
-            p.rows_per_thread = r;
-            p.width = width;
-            p.smem = (int)bytes;
-            return p;
-        }
+        if (L.smem == 0 || bytes > (size_t)L.smem || c > L.ctas) continue;
+        Plan p;
+        p.ctas = c;
+        p.rows_per_thread = r;
+        p.width = width;
+        p.smem = (int)bytes;
+        return p;
     }
     // beyond a cluster: one CTA per SM. Right-hand sides that do not fit together are solved
     // one after another; with ILU(0) that is slower than the graph engine's joint solve
     // (216,000 hexes, three right-hand sides, us per iteration: Jacobi 3 x 13.8 against 76,
     // ILU(0) 3 x 34 against 88).
+    const int sms = grid_ctas();
     for (int comps : {1, nrhs}) {
         if (max_ctas == 1 || (comps > 1 && precond == KCFD_PREC_ILU0)) break;
         const int joint = nrhs / comps;
         for (int r = 1; r <= 8; ++r) {
+            if (rows_on(sms) > kBlock * r) continue;
             const Limits L = limits(joint + 4, precond, r);
             size_t bytes = SIZE_MAX;
             dispatch(joint, precond, r, [&](auto n, auto p, auto rr) { bytes = Store<n(), p(), rr(), true>::bytes(width, nlev); });
-            if (L.smem == 0 || bytes > (size_t)L.smem || rows_on(L.ctas) > kBlock * r) continue;
+            if (L.smem == 0 || bytes > (size_t)L.smem) continue;
             Plan p;
             p.ctas = L.ctas;
             p.grid = true;
@@ -270,9 +280,10 @@ Plan plan_compact(int n, int width, int precond) {
     // leaves fewer shapes (launches) in a batch
     for (int c = 1; c <= kMaxCtas; c += c < 6 ? 1 : c < 12 ? 2 : 4)
         for (int r = c < 3 ? 1 : 8; r <= 8; ++r) {
+            if ((int64_t)c * kBlock * r < n) continue;
             const Limits L = limits(0, precond, r);
             const size_t bytes = (size_t)kBlock * r * (8 + 12 * (size_t)width) + 16;
-            if (L.ctas < c || bytes > (size_t)L.smem || (int64_t)c * kBlock * r < n) continue;
+            if (L.ctas < c || bytes > (size_t)L.smem) continue;
             Plan p;
             p.ctas = c;
             p.rows_per_thread = r;
