@@ -204,6 +204,13 @@ Limits limits(int nrhs, int precond, int r) {
     Plan p;
     p.smem = optin - (int)fa.sharedSizeBytes;
     if (nrhs > 4) {
+        // a cooperative launch needs all its CTAs resident together: one per SM at that much
+        int coop = 0, per_sm = 0;
+        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kBlock, p.smem) != cudaSuccess || per_sm < 1) {
+            cudaGetLastError();
+            return Limits();
+        }
         L.ctas = grid_ctas();
         L.smem = p.smem;
         return L;
