@@ -207,12 +207,10 @@ def outer_step_bytes(n, Fi, Fb, nnz, ndim, its_m, its_p, p_precond="amg", amg=No
 
 def solve_launches(solver, iters):
     """Kernels one solve launches: the persistent kernels and the on-chip solves launch
-    once (a system that may fit on chip counts as one: a lower bound where it does not);
-    the graph engine launches the value fill, init, final and the two copies plus, per
+    once; the graph engine launches the value fill, init, final and the two copies plus, per
     loop trip, the phase kernels (5), 2 (nlev - 1) ILU sweeps for each of phat and shat,
     or two V-cycles (4 kernels per level above the coarsest and the coarse solve)."""
-    from kcfd.solver import ON_CHIP_ROWS
-    if not solver.graph_engine or (solver.precond != "amg" and solver.n <= ON_CHIP_ROWS):
+    if solver.on_chip or not solver.graph_engine:
         return 1
     info = solver.info()
     body = 5
@@ -228,11 +226,10 @@ def setup_launches(solver, power_iters=8):
     """Kernels of one preconditioner set-up: Jacobi 1; ILU(0) at least 2 (one per level, or
     permute + factor; + 2 SELL fills on the graph engine beyond the chip); AMG per level
     above the coarsest 9 (level 0) or 10 + power iterations, and 2 for the coarsest."""
-    from kcfd.solver import ON_CHIP_ROWS
     if solver.precond == "jacobi":
         return 1
     if solver.precond == "ilu0":
-        return 2 + (2 if solver.graph_engine and solver.n > ON_CHIP_ROWS else 0)
+        return 2 + (2 if solver.graph_engine and not solver.on_chip else 0)
     if solver.precond == "amg":
         L = solver.info()["levels"]
         return (9 if L > 1 else 0) + max(0, L - 2) * (10 + power_iters) + 2
@@ -571,7 +568,7 @@ def c4_measure(count=C4_TOTAL, steps=1, warmup=1, mode="fp64", plain=True, plain
                restarts=20, world=1, rank=0):
     """The first `count` of the 1,024 C4 systems (cell counts log-uniform in [2e3, 2e5],
     seed 0; the same systems whatever the count) solved together: BiCGSTAB + Jacobi to
-    1e-8 per system, one persistent launch per size tier, a system whose rho or omega
+    1e-8 per system, one launch per size tier or on-chip shape, a system whose rho or omega
     breaks down restarted (up to `restarts` times). Returns the measurements: batched
     solves/s over converged systems, e2e with host buffers, the plain FP64 drop-in per
     system over a bounded prefix, the CPU scipy path over a bounded prefix."""
@@ -634,11 +631,19 @@ def c4_measure(count=C4_TOTAL, steps=1, warmup=1, mode="fp64", plain=True, plain
     byts = sum(_c4_bytes(int(n_sys[k]), int(nnz_sys[k]), int(its[k]), mixed) for k in range(len(mine)))
     launch = t / steps
     peak = measured_peak()
-    tiers = bs.tiers()
-    roof = {"bound": "hbm", "kernel": f"batch_cluster_kernel<MIXED={int(mixed)}, JACOBI> ({tiers['cluster']} systems on "
-                                      f"thread-block clusters of 2-{tiers['cluster_size']} CTAs graded by size) + "
-                                      f"batch_kernel<MIXED={int(mixed)}, JACOBI, 512 | 256> (one CTA per system), "
-                                      "largest first, one persistent launch per tier",
+    tiers, chip = bs.tiers(), bs.on_chip()
+    in_tiers = sum(1 for k in ("cluster", "big", "small") if tiers[k] > 0)
+    kernels = []
+    if chip["systems"]:
+        kernels.append(f"k_resident_batch ({chip['systems']} systems on chip, one cluster each, {chip['launches']} launches; "
+                       "their bytes are counted as if streamed)")
+    if tiers["cluster"]:
+        kernels.append(f"batch_cluster_kernel<MIXED={int(mixed)}, JACOBI> ({tiers['cluster']} systems on thread-block "
+                       f"clusters of 2-{tiers['cluster_size']} CTAs graded by size)")
+    if tiers["big"] or tiers["small"]:
+        kernels.append(f"batch_kernel<MIXED={int(mixed)}, JACOBI, 512 | 256> ({tiers['big'] + tiers['small']} systems, one "
+                       "CTA each)")
+    roof = {"bound": "hbm", "kernel": " + ".join(kernels) + ", largest first, one launch per tier or shape",
             "unit_of_work": "one launch solving all systems", "achieved": round(byts / launch / 1e9, 1),
             "peak": peak[0], "unit": "GB/s", "frac": round(byts / launch / 1e9 / peak[0], 3),
             "peak_source": peak[1], "traffic": None, "launch_ms": round(launch * 1e3, 3)}
@@ -721,8 +726,8 @@ def c4_measure(count=C4_TOTAL, steps=1, warmup=1, mode="fp64", plain=True, plain
             "ms_per_step": round(1e3 * t / steps, 3), "mixed": mixed, "clocks": clocks, "e2e": e2e,
             "roofline": roof, "plain_fp64_dropin": plain_d, "cpu_baseline": cpu_d,
             "batched_over_plain": round(value / plain_d["value"], 2) if plain_d else None,
-            "gpu_launches": (1 + sum(1 for k in ("cluster", "big", "small") if tiers[k] > 0)) * steps,
-            "tiers": tiers, "status_ok": int((st == 0).sum()), "breakdown": int((st == 2).sum()),
+            "gpu_launches": (chip["launches"] + in_tiers + (1 if in_tiers else 0)) * steps,
+            "tiers": {**tiers, "on_chip": chip["systems"]}, "status_ok": int((st == 0).sum()), "breakdown": int((st == 2).sum()),
             "converged": n_ok, "restarts_allowed": restarts, "max_true_relres": float(true_rel.max()),
             "krylov_iters": {"min": int(its.min()), "median": int(np.median(its)), "max": int(its.max())},
             "cells_this_rank": int(n_sys.sum()), "nnz_this_rank": int(nnz_sys.sum()),
@@ -731,7 +736,7 @@ def c4_measure(count=C4_TOTAL, steps=1, warmup=1, mode="fp64", plain=True, plain
                     "[2e3, 2e5], seed 0), diffusion (harmonic, Gamma log-uniform [0.1, 10]) + one Dirichlet side, "
                     "RHS N(0,1); batched " + ("FP32 BiCGSTAB + Jacobi with FP64 refinement" if mixed else
                                               "FP64 BiCGSTAB + Jacobi") +
-                    f", rtol 1e-8, breakdown restarts <= {restarts}, one persistent launch per size tier; value "
+                    f", rtol 1e-8, breakdown restarts <= {restarts}, one launch per size tier or on-chip shape; value "
                     "counts converged systems only"}
 
 

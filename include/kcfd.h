@@ -222,11 +222,12 @@ typedef struct {
                             conditioned systems, so only when asked for). Auto:
                             1 for n*nrhs <= 1024, 2 up to 40000 and for MIXED,
                             else 3. With the choice left so (lanes and block 0)
-                            a FP64 BiCGSTAB solve with Jacobi, ILU or no
+                            a BiCGSTAB solve with Jacobi, ILU or no
                             preconditioner whose system fits on chip runs there
-                            instead: in the shared memory and registers of a
-                            thread-block cluster, or of one CTA per SM (a
-                            cooperative launch). So does one that fits a single
+                            instead, FP64 also where MIXED was asked for: in
+                            the shared memory and registers of a thread-block
+                            cluster, or of one CTA per SM (a cooperative
+                            launch). So does an FP64 one that fits a single
                             CTA with team 1, lanes <= 1 and block 0 or 256.
                             KCFD_ENGINE_EAGER=1 in the environment at creation
                             launches the engine's kernels from a host loop
@@ -384,8 +385,10 @@ void kcfd_batch_destroy(kcfd_batch* b);
 /* info[0..3] = nsys, total rows, total entries, CTAs per launch */
 int  kcfd_batch_info(const kcfd_batch* b, int64_t* info);
 /* tiers[5]: systems in the cluster, big and small tiers, clusters launched, CTAs
- * per cluster.                                                                     */
+ * per cluster. Systems solved on chip are in none of them: counts2[0] of those, in
+ * counts2[1] launches.                                                             */
 int  kcfd_batch_tiers(const kcfd_batch* b, int32_t* tiers);
+int  kcfd_batch_on_chip(const kcfd_batch* b, int32_t* counts2);
 /* vals64, rhs, x: packed device arrays (system s at its row / entry offset); x holds
  * x0 on entry. iters/relres/status: device arrays of nsys entries.                 */
 int  kcfd_batch_solve(kcfd_batch* b, const double* vals64, const double* rhs, double* x, int32_t* iters,
@@ -545,6 +548,9 @@ int kcfd_solver_error(kcfd_solver* s, int32_t* err, void* stream);
  * grid, 3 graph engine), info[1] lanes per row, info[2] threads per CTA, info[3]
  * ILU(0) levels (1 without ILU). No reference counterpart (diagnostics).         */
 int kcfd_solver_info(const kcfd_solver* s, int32_t* info4);
+/* Where the handle solves: *ctas CTAs hold its system on chip (one kernel, whatever the
+ * team: of info's values it then uses none), or 0: it solves as info's team.         */
+int kcfd_solver_on_chip(const kcfd_solver* s, int32_t* ctas);
 
 /* ------------------------------------------------ two-fluid system set ----- */
 /* The pieces of the Euler-Euler model (models/two_fluid.py, models/closure.py) that

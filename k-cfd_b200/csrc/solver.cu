@@ -2521,6 +2521,12 @@ int kcfd_solver_info(const kcfd_solver* s, int32_t* info4) {
     return KCFD_OK;
 }
 
+int kcfd_solver_on_chip(const kcfd_solver* s, int32_t* ctas) {
+    KCFD_REQUIRE(s && ctas, "kcfd_solver_on_chip: NULL argument");
+    *ctas = s->res.ctas;
+    return KCFD_OK;
+}
+
 int kcfd_solver_error(kcfd_solver* s, int32_t* err, void* stream) {
     KCFD_REQUIRE(s && err, "kcfd_solver_error: NULL argument");
     KCFD_CUDA(cudaMemcpyAsync(err, s->err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
@@ -2583,7 +2589,6 @@ struct kcfd_batch {
     };
     std::vector<Chip> chip;
     int nchip = 0;
-    int rep_huge = 0, rep_big = 0, rep_cl[kMaxClTiers] = {}, rep_ncl[kMaxClTiers] = {};  // by row count, chip ones included
 };
 
 namespace {
@@ -2798,14 +2803,11 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
         return on_chip(x) ? shape(x) > shape(y) : tier(x) < tier(y);
     });
     for (int s = 0; s < nsys; ++s) {
-        const int t = tier(s);
-        b->rep_huge += t < nt ? 1 : 0;
-        b->rep_big += t == nt ? 1 : 0;
-        if (t < nt) b->rep_cl[t]++;
         if (on_chip(s)) {
             b->nchip++;
             continue;
         }
+        const int t = tier(s);
         if (t < nt) b->cl_n[t]++;
         b->nhuge += t < nt ? 1 : 0;
         b->nbig += t == nt ? 1 : 0;
@@ -2814,7 +2816,6 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
         b->cl_first[t] = first;
         first += b->cl_n[t];
         b->cl_ncl[t] = std::min(b->cl_n[t], ncl_max[t]);
-        b->rep_ncl[t] = std::min(b->rep_cl[t], ncl_max[t]);
     }
     for (int q = nsys - b->nchip; q < nsys; ++q) {
         const int x = order[q];
@@ -2826,7 +2827,7 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
     int per_sm = 0, per_sm_big = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_ptr(mixed, b->o.precond, false), 256, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_big, batch_kernel_ptr(mixed, b->o.precond, true), 512, 0);
-    const int nsmall = nsys - b->rep_big - b->rep_huge;
+    const int nsmall = nsys - b->nchip - b->nbig - b->nhuge;
     b->grid = std::max(1, std::min(std::max(nsmall, 1), std::max(1, per_sm) * sms));
     b->grid_big = std::max(1, std::min(std::max(b->nbig, 1), std::max(1, per_sm_big) * sms));
     bool ok = cudaMalloc(&b->sys, nsys * sizeof(BatchSys)) == cudaSuccess &&
@@ -2896,15 +2897,22 @@ int kcfd_batch_info(const kcfd_batch* b, int64_t* info) {
 
 int kcfd_batch_tiers(const kcfd_batch* b, int32_t* tiers) {
     KCFD_REQUIRE(b && tiers, "kcfd_batch_tiers: NULL argument");
-    tiers[0] = b->rep_huge;
-    tiers[1] = b->rep_big;
-    tiers[2] = b->nsys - b->rep_huge - b->rep_big;
+    tiers[0] = b->nhuge;
+    tiers[1] = b->nbig;
+    tiers[2] = b->nsys - b->nchip - b->nhuge - b->nbig;
     tiers[3] = 0;
     tiers[4] = 0;
     for (int t = 0; t < b->ntier; ++t) {
-        tiers[3] += b->rep_cl[t] > 0 ? b->rep_ncl[t] : 0;
-        if (b->rep_cl[t] > 0) tiers[4] = std::max(tiers[4], b->cl_size[t]);
+        tiers[3] += b->cl_n[t] > 0 ? b->cl_ncl[t] : 0;
+        if (b->cl_n[t] > 0) tiers[4] = std::max(tiers[4], b->cl_size[t]);
     }
+    return KCFD_OK;
+}
+
+int kcfd_batch_on_chip(const kcfd_batch* b, int32_t* counts2) {
+    KCFD_REQUIRE(b && counts2, "kcfd_batch_on_chip: NULL argument");
+    counts2[0] = b->nchip;
+    counts2[1] = (int)b->chip.size();
     return KCFD_OK;
 }
 

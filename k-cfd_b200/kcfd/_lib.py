@@ -88,6 +88,7 @@ SIGNATURES = {
     "kcfd_solver_solve": (i32, [vp, C.POINTER(Csr), vp, vp, vp, vp, vp, vp]),
     "kcfd_solver_error": (i32, [vp, P_i32, vp]),
     "kcfd_solver_info": (i32, [vp, P_i32]),
+    "kcfd_solver_on_chip": (i32, [vp, P_i32]),
     "kcfd_solver_apply_precond": (i32, [vp, C.POINTER(Csr), vp, vp, vp]),
     "kcfd_solver_amg": (i32, [vp, C.POINTER(vp)]),
     "kcfd_amg_create": (i32, [C.POINTER(Csr), C.POINTER(AmgOpts), C.POINTER(vp)]),
@@ -132,6 +133,7 @@ SIGNATURES = {
     "kcfd_batch_destroy": (None, [vp]),
     "kcfd_batch_info": (i32, [vp, P_i64]),
     "kcfd_batch_tiers": (i32, [vp, P_i32]),
+    "kcfd_batch_on_chip": (i32, [vp, P_i32]),
     "kcfd_selftest_barrier": (i32, [i32, i32, i64, vp, vp, vp]),
     "kcfd_selftest_on_chip": (i32, [i32, i32, i64, i32, i64, vp, vp, vp]),
     "kcfd_graph_capture_begin": (i32, [vp]),

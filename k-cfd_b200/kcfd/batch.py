@@ -77,10 +77,17 @@ class BatchSolver:
         self.status = torch.zeros(self.nsys, dtype=torch.int32, device=dev)
 
     def tiers(self):
-        """dict(cluster, big, small, clusters, cluster_size): systems per tier, clusters launched."""
+        """dict(cluster, big, small, clusters, cluster_size): systems per tier, clusters launched.
+        Systems solved on chip are in none of the tiers (on_chip)."""
         v = np.zeros(5, dtype=np.int32)
         _lib.check(_lib.lib().kcfd_batch_tiers(self._h, v.ctypes.data_as(_lib.P_i32)), "kcfd_batch_tiers")
         return dict(zip(("cluster", "big", "small", "clusters", "cluster_size"), (int(t) for t in v)))
+
+    def on_chip(self):
+        """dict(systems, launches): systems solved on chip, and the launches (one per shape) they take."""
+        v = np.zeros(2, dtype=np.int32)
+        _lib.check(_lib.lib().kcfd_batch_on_chip(self._h, v.ctypes.data_as(_lib.P_i32)), "kcfd_batch_on_chip")
+        return {"systems": int(v[0]), "launches": int(v[1])}
 
     def __del__(self):
         h = getattr(self, "_h", None)

@@ -185,9 +185,16 @@ class Solver:
         return {"team": int(v[0]), "lanes": int(v[1]), "block": int(v[2]), "levels": int(v[3])}
 
     @property
+    def on_chip(self):
+        """CTAs that hold the system on chip, 0 when it is solved by info()'s team."""
+        c = C.c_int32(0)
+        _lib.check(_lib.lib().kcfd_solver_on_chip(self._h, C.byref(c)), "kcfd_solver_on_chip")
+        return c.value
+
+    @property
     def graph_engine(self):
         """True for a handle of team 3: its solves run as the handle's own CUDA graph, or
-        on chip where the system fits. The graph is not nested into an enclosing
+        on chip where the system fits (on_chip). The graph is not nested into an enclosing
         stream capture (there such a solve runs on the persistent grid kernel), so
         callers keep it outside their captures."""
         return self.info()["team"] == 3
