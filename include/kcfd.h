@@ -551,6 +551,10 @@ int kcfd_solver_info(const kcfd_solver* s, int32_t* info4);
 /* Where the handle solves: *ctas CTAs hold its system on chip (one kernel, whatever the
  * team: of info's values it then uses none), or 0: it solves as info's team.         */
 int kcfd_solver_on_chip(const kcfd_solver* s, int32_t* ctas);
+/* The same for a handle that does not exist yet: BiCGSTAB with an automatic launch shape on a
+ * matrix of n rows of at most `width` entries; ILU(0) with the given level of each row.   */
+int kcfd_on_chip_ctas(int32_t n, int32_t width, int32_t nrhs, int32_t precond, const int32_t* level_of_row_host,
+                      int32_t* ctas);
 
 /* ------------------------------------------------ two-fluid system set ----- */
 /* The pieces of the Euler-Euler model (models/two_fluid.py, models/closure.py) that

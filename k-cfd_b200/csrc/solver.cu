@@ -2521,6 +2521,28 @@ int kcfd_solver_info(const kcfd_solver* s, int32_t* info4) {
     return KCFD_OK;
 }
 
+int kcfd_on_chip_ctas(int32_t n, int32_t width, int32_t nrhs, int32_t precond, const int32_t* level_of_row_host,
+                      int32_t* ctas) {
+    KCFD_REQUIRE(ctas && n > 0 && width > 0 && nrhs >= 1 && nrhs <= 3, "kcfd_on_chip_ctas: bad arguments");
+    KCFD_REQUIRE(precond >= 0 && precond <= 3, "kcfd_on_chip_ctas: bad precond");
+    KCFD_REQUIRE(precond != KCFD_PREC_ILU0 || level_of_row_host, "kcfd_on_chip_ctas: ILU(0) needs the rows' levels");
+    *ctas = 0;
+    if (precond == KCFD_PREC_AMG) return KCFD_OK;
+    std::vector<int> lev = {0, n};
+    if (precond == KCFD_PREC_ILU0) {
+        lev.assign(1, 0);
+        for (int i = 0; i < n; ++i) {
+            const int l = level_of_row_host[i];
+            KCFD_REQUIRE(l >= 0 && l < n, "kcfd_on_chip_ctas: level out of range at row %d", i);
+            if ((int)lev.size() < l + 2) lev.resize(l + 2, 0);
+            lev[l + 1]++;
+        }
+        for (size_t l = 1; l < lev.size(); ++l) lev[l] += lev[l - 1];
+    }
+    *ctas = res::plan(width, nrhs, precond, lev, res::kMaxCtas).ctas;
+    return KCFD_OK;
+}
+
 int kcfd_solver_on_chip(const kcfd_solver* s, int32_t* ctas) {
     KCFD_REQUIRE(s && ctas, "kcfd_solver_on_chip: NULL argument");
     *ctas = s->res.ctas;

@@ -89,6 +89,7 @@ SIGNATURES = {
     "kcfd_solver_error": (i32, [vp, P_i32, vp]),
     "kcfd_solver_info": (i32, [vp, P_i32]),
     "kcfd_solver_on_chip": (i32, [vp, P_i32]),
+    "kcfd_on_chip_ctas": (i32, [i32, i32, i32, i32, vp, P_i32]),
     "kcfd_solver_apply_precond": (i32, [vp, C.POINTER(Csr), vp, vp, vp]),
     "kcfd_solver_amg": (i32, [vp, C.POINTER(vp)]),
     "kcfd_amg_create": (i32, [C.POINTER(Csr), C.POINTER(AmgOpts), C.POINTER(vp)]),

@@ -205,22 +205,25 @@ class Solver:
         return e.value
 
 
-# rows up to which a MIXED system may fit on chip (one CTA per SM, 8 rows a thread)
-ON_CHIP_ROWS = 303104
+def on_chip_ctas(csr, precond, nrhs=1, levels=None):
+    """CTAs that would hold csr's system on chip, 0 where it does not fit (kcfd_on_chip_ctas);
+    ILU(0) with the given row levels."""
+    lev = None if levels is None else np.ascontiguousarray(levels, dtype=np.int32)
+    width = int((csr.indptr[1:] - csr.indptr[:-1]).max())
+    c = C.c_int32(0)
+    _lib.check(_lib.lib().kcfd_on_chip_ctas(csr.n, width, nrhs, _lib.PREC[precond], _lib.ptr(lev), C.byref(c)),
+               "kcfd_on_chip_ctas")
+    return c.value
 
 
-def mixed_handle(csr, team=0, nrhs=1, **kw):
+def mixed_handle(csr, team=0, nrhs=1, precond="jacobi", levels=None, lanes=0, **kw):
     """A MIXED Solver: on chip where the system fits (FP64 there), else the graph engine's
     FP32 form above 40,000 unknowns, else the persistent kernel's FP32 inner iterations.
-    An explicit team is taken as it is."""
-    kw["mode"] = _lib.MODE_MIXED
-    if team == 0 and csr.n * nrhs > 40000:
-        if csr.n <= ON_CHIP_ROWS:
-            s = Solver(csr, nrhs=nrhs, **kw)
-            if s.info()["team"] == 3:
-                return s
+    An explicit team is taken as it is, and an explicit number of lanes keeps the system off
+    the chip."""
+    if team == 0 and csr.n * nrhs > 40000 and (lanes > 0 or not on_chip_ctas(csr, precond, nrhs, levels)):
         team = 3
-    return Solver(csr, team=team, nrhs=nrhs, **kw)
+    return Solver(csr, team=team, nrhs=nrhs, precond=precond, levels=levels, lanes=lanes, mode=_lib.MODE_MIXED, **kw)
 
 
 class DeviceGraph:

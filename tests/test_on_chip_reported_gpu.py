@@ -41,3 +41,29 @@ def test_batch():
         t = B.tiers()
         assert B.on_chip() == {"systems": 0, "launches": 0}
         assert t["cluster"] + t["big"] + t["small"] == len(sizes)
+
+
+@pytest.mark.parametrize("N,prec,nrhs,lanes,chip,team", [(30, "jacobi", 3, 0, True, 3), (36, "ilu0", 1, 0, True, 3),
+                                                         (62, "ilu0", 1, 0, False, 3), (36, "jacobi", 1, 4, False, 3),
+                                                         (20, "jacobi", 1, 0, True, 2)])
+def test_mixed_handle_makes_one(monkeypatch, N, prec, nrhs, lanes, chip, team):
+    """The handle is made once, also where the system does not fit; the plan agrees with the handle."""
+    from scipy import sparse
+    import kcfd.solver as ks
+    T, I = sparse.diags([-np.ones(N - 1), np.full(N, 2.1), -np.ones(N - 1)], [-1, 0, 1]), sparse.identity(N)
+    A = (sparse.kron(sparse.kron(T, I), I) + sparse.kron(sparse.kron(I, T), I) + sparse.kron(sparse.kron(I, I), T)).tocsr()
+    d = ks.DeviceCSR.from_scipy(A, fp32=True)
+    i = np.arange(N ** 3)
+    levels = ((i + i // N + i // N ** 2) % 2).astype(np.int32) if prec == "ilu0" else None
+    made = []
+
+    class Counted(ks.Solver):
+        def __init__(self, *a, **kw):
+            made.append(1)
+            super().__init__(*a, **kw)
+
+    monkeypatch.setattr(ks, "Solver", Counted)
+    s = ks.mixed_handle(d, precond=prec, nrhs=nrhs, levels=levels, lanes=lanes, rtol=1e-8)
+    assert len(made) == 1
+    assert (s.on_chip > 0) == chip and s.info()["team"] == team
+    assert lanes or ks.on_chip_ctas(d, prec, nrhs, levels) == s.on_chip
