@@ -429,7 +429,7 @@ struct MomentumOp {
         return d;
     }
     __device__ double apply(const CellFace& c, const Data& d, Acc& a) const {
-        const double pf = 0.5 * (a.p + d.p), s = c.own ? -a.a : a.a;  // the own p on a boundary face
+        const double pf = c.in ? 0.5 * (a.p + d.p) : a.p, s = c.own ? -a.a : a.a;
 #pragma unroll
         for (int k = 0; k < 3; ++k) a.s[k] += s * pf * d.n[k] * d.A;
         return 0.0;
@@ -521,9 +521,10 @@ struct CorrectOp {
         for (int k = 0; k < D; ++k) d.n[k] = __ldg(m.normal + c.f * D + k);
         return d;
     }
-    __device__ double apply(const CellFace&, const Data& d, Acc& a) const {
+    __device__ double apply(const CellFace& c, const Data& d, Acc& a) const {
         // pp[neighbour] - pp[owner] is added on the owner side; on the neighbour side the
-        // same product is negated twice; 0 on a boundary face
+        // same product is negated twice
+        if (!c.in) return 0.0;
         const double dp = d.pp - a.pp;
 #pragma unroll
         for (int k = 0; k < D; ++k) a.s[k] += dp * d.n[k] * d.A;
