@@ -165,7 +165,10 @@ struct ClusterTeam {
     // CTA alike, when none expired. No CTA returns while another may gather from it.
     __device__ bool settle(bool ok) const {
         if (size == 1) return ok;
-        if (threadIdx.x == 0) tell(&sh->settled[rank]);
+        if (threadIdx.x == 0) {
+            if (!ok) tell(&sh->any_fail);
+            tell(&sh->settled[rank]);
+        }
         if (ok) {
             sync();  // the same barrier for all CTAs whose waits were met; the others meet it too
             return *(volatile int*)&sh->any_fail == 0;
@@ -228,10 +231,7 @@ struct ClusterTeam {
                 if (ok) break;
                 if (poll % 16 == 0 && (*(volatile int*)&sh->any_fail != 0 || clock64() - t0 > budget)) break;
             }
-            if (!ok) {
-                tell(&sh->any_fail);
-                sh->fail = 1;
-            }
+            if (!ok) sh->fail = 1;
             __syncwarp();
             s = tree_sum<kMaxCtas>(sh->part[h] + q * kMaxCtas);
         }
