@@ -2332,7 +2332,6 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
     bool ok = upload(&s->lev_ptr, lptr);
     if (s->res.ctas == 0) ok = ok && cudaMalloc(&s->work, 9 * len * vsz) == cudaSuccess;
     else if (s->res.scratch > 0) ok = ok && cudaMalloc(&s->work, s->res.scratch * sizeof(double)) == cudaSuccess;
-    if (ok && s->res.scratch > 0) ok = cudaMemset(s->work, 0, s->res.scratch * sizeof(double)) == cudaSuccess;
     if (mixed) ok = ok && cudaMalloc(&s->r64, len * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&s->bar, 2 * sizeof(unsigned)) == cudaSuccess;
     ok = ok && cudaMalloc(&s->err, sizeof(int)) == cudaSuccess;
@@ -2363,6 +2362,12 @@ int kcfd_solver_create(const kcfd_csr_t* A, const kcfd_solver_opts_t* opts, cons
             free_solver(s);
             return e;
         }
+    }
+    // the first solve may come on a stream that does not wait for the zeroing above
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+        free_solver(s);
+        set_error("kcfd_solver_create: device initialisation failed");
+        return KCFD_CUDA_ERROR;
     }
     *out = s;
     return KCFD_OK;
