@@ -139,7 +139,8 @@ def measured_peak():
 # on the 128^3 cavity, from an ncu launch list of one solve on the graph engine
 # (KCFD_ENGINE_EAGER=1, every kernel of the solve captured, one pass each), divided
 # by the solve's Krylov count; the roofline's traffic is this times the timed solve's
-# count. Keyed by preconditioner; None where no capture was made.
+# count. Keyed by preconditioner; None where no capture was made. Taken before the vector
+# kernels ran over flat values, which read and write the same vectors.
 NCU_P_ITER_DRAM_BYTES_128 = {"ilu0": 857019136, "amg": 2471459375}
 
 

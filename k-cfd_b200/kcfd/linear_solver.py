@@ -20,7 +20,7 @@ device failure raises instead of falling back to the CPU. Semantics kept:
   * method='direct': the device has no sparse LU; BiCGSTAB + ILU(0) to a relative
     residual of 1e-12 stands in for spsolve (documented difference). A matrix without
     ILU levels of its own is coloured first: natural-order levels are some hundred
-    short dependent steps per sweep (5,000 triangles, whole call: 84 ms against 7.4 ms coloured);
+    short dependent steps per sweep (5,000 triangles, whole call: 84 ms against 8 ms coloured);
     they are the second try, from x0 again, where the coloured factor does not reach that
     residual in a bounded number of iterations, and the only one for chain-like matrices.
 system may be the reference's FVMSystem (anything with .to_sparse() and .rhs), a
@@ -130,8 +130,8 @@ def _direct_tries(d, its):
 def _residual_met(d, b, x):
     """||b - A x|| <= DIRECT_RTOL ||b||, or within the rounding of the residual itself (rows of some
     eight entries: 8 u (|A| |x| + |b|)), below which no solution can be told from another."""
-    norm = float(b.norm())
-    res = float((b - d.spmv(x)).norm())
+    torch = _lib.require_cuda()
+    norm, res = torch.stack((b.norm(), (b - d.spmv(x)).norm())).tolist()
     if res <= DIRECT_RTOL * norm:
         return True
     floor = DeviceCSR(d.indptr, d.indices, d.vals64.abs()).spmv(x.abs()) + b.abs()
