@@ -12,7 +12,7 @@
 // each step issues the loads of B faces before it uses any, and both slots of a face are
 // loaded so that the row entry does not wait for the owner. (4 or 8 lanes per cell, a face
 // per lane, coalesce better but keep fewer loads in flight: 97-183 us for the operators of
-// operators.cu on 96^3 hexes against 57-70.)
+// operators.cu on 96^3 hexes against 54-67.)
 #pragma once
 #include <cuda_runtime.h>
 
@@ -65,11 +65,11 @@ __global__ void __launch_bounds__(256) k_by_cell(kcfd_dmesh_t m, Op op) {
             d[u] = op.load(m, i, c[u], acc);
         }
         if constexpr (Op::kOff) {
-            bool shared = false;  // two faces to the same cell (or the padding of a last step)
+            bool shared = false;  // two faces to the same cell (not the padding of a last step)
 #pragma unroll
             for (int u = 1; u < B; ++u)
 #pragma unroll
-                for (int w = 0; w < u; ++w) shared |= c[u].in && on[w] == on[u];
+                for (int w = 0; w < u; ++w) shared |= c[u].in && e + u < e1 && on[w] == on[u];
             if (shared) {
 #pragma unroll
                 for (int u = 0; u < B; ++u) {
@@ -95,8 +95,9 @@ __global__ void __launch_bounds__(256) k_by_cell(kcfd_dmesh_t m, Op op) {
 template <class Op>
 void by_cell(const kcfd_dmesh_t* m, const Op& op, cudaStream_t st) {
     if (m->n_cells <= 0) return;
-    // three faces a step: 32-62 registers. On 96^3 hexes (diffusion, convection, MUSCL): 70, 57
-    // and 66 us; two faces 70, 105 and 66; four 74, 57 and 76; six 84, 88 and 80
+    // three faces a step: 32-62 registers. On 96^3 hexes (diffusion, convection, MUSCL): 67, 54
+    // and 66 us. The sizes against one another, measured before a step looked for shared entries:
+    // three 70, 57 and 66; two 70, 105 and 66; four 74, 57 and 76; six 84, 88 and 80
     k_by_cell<3, Op><<<(m->n_cells + 255) / 256, 256, 0, st>>>(*m, op);
 }
 

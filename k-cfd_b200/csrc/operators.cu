@@ -13,7 +13,7 @@
 // under_relax reads diag (which a caller may floor on its own, as the two-fluid model
 // does). Face operators run by cell (by_cell.cuh), or, on a mesh without cell lists, one
 // launch per face colour (conflict-free scatter). On 96^3 jittered hexes (FP64, cold L2;
-// colours, then by cell): diffusion 171 and 70 us, convection 177 and 57, MUSCL 91 and 66,
+// colours, then by cell): diffusion 173 and 67 us, convection 181 and 54, MUSCL 91 and 66,
 // boundary conditions 26 and 16; on 500,000 triangles 73 and 33, 67 and 23, 46 and 29.
 #include <cuda_runtime.h>
 
