@@ -2581,7 +2581,7 @@ struct kcfd_batch {
     kcfd_batch_opts_t o;
     int nsys = 0;
     long long n_total = 0, nnz_total = 0;
-    int grid = 0;
+    int grid = 0, prep_grid = 0;
     BatchSys* sys = nullptr;
     int* order = nullptr;
     int* queue = nullptr;
@@ -2855,6 +2855,7 @@ int kcfd_batch_create(int32_t nsys, const int32_t* n, const int32_t* nnz, const 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_ptr(mixed, b->o.precond, false), 256, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_big, batch_kernel_ptr(mixed, b->o.precond, true), 512, 0);
     const int nsmall = nsys - b->nchip - b->nbig - b->nhuge;
+    b->prep_grid = 4 * std::max(1, per_sm) * sms;  // its CTAs take the tiers' systems in turn, whatever the tier
     b->grid = std::max(1, std::min(std::max(nsmall, 1), std::max(1, per_sm) * sms));
     b->grid_big = std::max(1, std::min(std::max(b->nbig, 1), std::max(1, per_sm_big) * sms));
     bool ok = cudaMalloc(&b->sys, nsys * sizeof(BatchSys)) == cudaSuccess &&
@@ -2983,7 +2984,7 @@ int kcfd_batch_solve(kcfd_batch* b, const double* vals64, const double* rhs, dou
     if (b->nhuge > 0) KCFD_CUDA(cudaMemsetAsync(b->cerr, 0, sizeof(int), st));
     B.nq = b->nsys - b->nchip;  // the on-chip kernel sets its systems up itself
     void* args[] = {&B};
-    const int pgrid = std::max(1, std::min(B.nq, 4 * b->grid));
+    const int pgrid = std::max(1, std::min(B.nq, b->prep_grid));
     if (B.nq > 0)
         KCFD_CUDA(cudaLaunchKernel(B.mixed ? (void*)batch_prep_kernel<1> : (void*)batch_prep_kernel<0>, dim3(pgrid),
                                    dim3(256), args, 0, st));
